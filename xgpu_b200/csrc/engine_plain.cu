@@ -5,11 +5,12 @@
 // shared_transfer_4_dp4a.cuh:99-164).  The arithmetic per thread is the same:
 // each thread owns a 2x2 block of stations (rows i, i+1 x columns j, j+1) and
 // all 4 polarisation products of each, i.e. 16 complex visibilities.
-//   FP32: 32 float accumulators; per sample and visibility the two products
-//         of the real (and of the imaginary) part are summed exactly and the
-//         sum is added with one rounding, as xGPU's float engine does
-//         (omp_xengine.c:24-28), so the sums equal its own bit for bit:
-//         3 FP32 instructions per component, 96 per sample.
+//   FP32: 32 float sums; per sample and visibility the two products of the
+//         real (and of the imaginary) part are summed exactly and the sum is
+//         added with one rounding, as xGPU's float engine does
+//         (omp_xengine.c:24-28), so the sums equal its own bit for bit.  While
+//         no sum can pass 2^24 those additions are exact and dp4a does them;
+//         from there on 3 FP32 instructions per component, 96 per sample.
 //   dp4a: 48 int32 accumulators (re, im1, im2 as in kernel.cuh:464-479,574),
 //         64 dp4a per group of 4 samples.
 // What changes is the data path.  xGPU fetches one sample at a time through
@@ -68,7 +69,8 @@ __device__ __forceinline__ int station_of_slot(int q) { return q < 16 ? 2 * q : 
 __device__ __forceinline__ int row_station_of_slot(int q) { return q < 8 ? 2 * q : 2 * (q - 8) + 1; }
 
 struct Params {
-  CUtensorMap map;  // the input, boxes of 128 bytes x one chunk of samples
+  CUtensorMap map;        // the input, boxes of 128 bytes x 64 samples (one dp4a chunk)
+  CUtensorMap map_float;  // FP32 engine: the same in boxes of 32 samples (float phase)
   int n, f;
   int t0, tcount;
   long long nbaseline;
@@ -88,11 +90,12 @@ struct Params {
 // column block's 32 stations.
 template <int NT>
 __device__ __forceinline__ void issue_panels(uint8_t (*raw)[NT * kRowBytes], uint32_t bar,
-                                             const Params &p, int f, int rb, int cb, int tb) {
+                                             const Params &p, const CUtensorMap &map, int f, int rb,
+                                             int cb, int tb) {
   if (p.stall) return;
   tc::mbar_expect_tx(bar, 2 * NT * kRowBytes);
-  tc::tma_load_3d(tc::smem_u32(raw[0]), &p.map, bar, rb * kRows * 4, f, tb);
-  tc::tma_load_3d(tc::smem_u32(raw[1]), &p.map, bar, cb * kRowBytes, f, tb);
+  tc::tma_load_3d(tc::smem_u32(raw[0]), &map, bar, rb * kRows * 4, f, tb);
+  tc::tma_load_3d(tc::smem_u32(raw[1]), &map, bar, cb * kRowBytes, f, tb);
 }
 
 // A panel that never arrived (bounded wait expired): record it and leave
@@ -137,6 +140,41 @@ __device__ __forceinline__ void to_words(const uint8_t *raw, int4 *words) {
     o.z = (int)__byte_perm(hi01, hi23, 0x5410);  // Y re
     o.w = (int)__byte_perm(hi01, hi23, 0x7632);  // Y im
     words[g * kSlots + q] = o;
+  }
+}
+
+// One converted chunk into the thread's 2x2 tile: re, and the two halves of im
+// (im = i1 - i2) kept apart, as -128 has no int8 negation.
+__device__ __forceinline__ void dp4a_chunk(const int4 *wrow, const int4 *wcol, int ty, int tx,
+                                           int (&re)[2][2][2][2], int (&i1)[2][2][2][2],
+                                           int (&i2)[2][2][2][2]) {
+#pragma unroll 1
+  for (int g = 0; g < kGroups; ++g) {
+    int4 r[2], c[2];
+    r[0] = wrow[g * kRows + ty];
+    r[1] = wrow[g * kRows + 8 + ty];
+    c[0] = wcol[g * kBlk + tx];
+    c[1] = wcol[g * kBlk + 16 + tx];
+    // Four sweeps over the 16 visibilities of the 2x2 tile, so that the two
+    // dp4a of one real part are 48 instructions apart, not back to back.
+#pragma unroll
+    for (int sweep = 0; sweep < 4; ++sweep)
+#pragma unroll
+      for (int rs = 0; rs < 2; ++rs)
+#pragma unroll
+        for (int cs = 0; cs < 2; ++cs) {
+          const int ar[2] = {r[rs].x, r[rs].z}, ai[2] = {r[rs].y, r[rs].w};
+          const int br[2] = {c[cs].x, c[cs].z}, bi[2] = {c[cs].y, c[cs].w};
+#pragma unroll
+          for (int p1 = 0; p1 < 2; ++p1)
+#pragma unroll
+            for (int p2 = 0; p2 < 2; ++p2) {
+              if (sweep == 0) re[rs][cs][p1][p2] = dp4a(ar[p1], br[p2], re[rs][cs][p1][p2]);
+              if (sweep == 1) i1[rs][cs][p1][p2] = dp4a(ai[p1], br[p2], i1[rs][cs][p1][p2]);
+              if (sweep == 2) i2[rs][cs][p1][p2] = dp4a(ar[p1], bi[p2], i2[rs][cs][p1][p2]);
+              if (sweep == 3) re[rs][cs][p1][p2] = dp4a(ai[p1], bi[p2], re[rs][cs][p1][p2]);
+            }
+        }
   }
 }
 
@@ -193,7 +231,7 @@ __global__ void __launch_bounds__(kThreads, 5) xengine_dp4a_kernel(const __grid_
     tc::mbar_init(bar0, 1);
     tc::mbar_init(bar0 + 8, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    issue_panels<kTcD>(raw[0], bar0, p, f, rb, cb, tbeg);
+    issue_panels<kTcD>(raw[0], bar0, p, p.map, f, rb, cb, tbeg);
   }
   __syncthreads();
 
@@ -201,7 +239,7 @@ __global__ void __launch_bounds__(kThreads, 5) xengine_dp4a_kernel(const __grid_
     const int buf = ch & 1;
     // Chunk ch+1 goes into the other buffer, free since the end of chunk ch-1.
     if (threadIdx.x == 0 && ch + 1 < nchunks)
-      issue_panels<kTcD>(raw[buf ^ 1], bar0 + 8 * (buf ^ 1), p, f, rb, cb,
+      issue_panels<kTcD>(raw[buf ^ 1], bar0 + 8 * (buf ^ 1), p, p.map, f, rb, cb,
                          tbeg + (ch + 1) * kTcD);
     const bool got = tc::mbar_wait(bar0 + 8 * buf, (ch >> 1) & 1, nullptr);
     if (__syncthreads_or(!got)) {
@@ -212,34 +250,7 @@ __global__ void __launch_bounds__(kThreads, 5) xengine_dp4a_kernel(const __grid_
     to_words<kRows>(raw[buf][0], wrow);
     to_words<kBlk>(raw[buf][1], wcol);
     __syncthreads();
-#pragma unroll 1
-    for (int g = 0; g < kGroups; ++g) {
-      int4 r[2], c[2];
-      r[0] = wrow[g * kRows + ty];
-      r[1] = wrow[g * kRows + 8 + ty];
-      c[0] = wcol[g * kBlk + tx];
-      c[1] = wcol[g * kBlk + 16 + tx];
-      // Four sweeps over the 16 visibilities of the 2x2 tile, so that the two
-      // dp4a of one real part are 48 instructions apart, not back to back.
-#pragma unroll
-      for (int sweep = 0; sweep < 4; ++sweep)
-#pragma unroll
-        for (int rs = 0; rs < 2; ++rs)
-#pragma unroll
-          for (int cs = 0; cs < 2; ++cs) {
-            const int ar[2] = {r[rs].x, r[rs].z}, ai[2] = {r[rs].y, r[rs].w};
-            const int br[2] = {c[cs].x, c[cs].z}, bi[2] = {c[cs].y, c[cs].w};
-#pragma unroll
-            for (int p1 = 0; p1 < 2; ++p1)
-#pragma unroll
-              for (int p2 = 0; p2 < 2; ++p2) {
-                if (sweep == 0) re[rs][cs][p1][p2] = dp4a(ar[p1], br[p2], re[rs][cs][p1][p2]);
-                if (sweep == 1) i1[rs][cs][p1][p2] = dp4a(ai[p1], br[p2], i1[rs][cs][p1][p2]);
-                if (sweep == 2) i2[rs][cs][p1][p2] = dp4a(ar[p1], bi[p2], i2[rs][cs][p1][p2]);
-                if (sweep == 3) re[rs][cs][p1][p2] = dp4a(ai[p1], bi[p2], re[rs][cs][p1][p2]);
-              }
-          }
-    }
+    dp4a_chunk(wrow, wcol, ty, tx, re, i1, i2);
     __syncthreads();
   }
 
@@ -297,12 +308,28 @@ __global__ void __launch_bounds__(kThreads, 5) xengine_dp4a_kernel(const __grid_
 }
 
 // ---------------------------------------------------------------- FP32 ----
-// The FP32 engine may not split time (its sums keep xGPU's order); the small
-// blocks balance its SMs.
-constexpr int kTcF = 32;                         // samples per chunk
+// xGPU's float sums (omp_xengine.c:24-28) in two phases, with the same bits.
+// A sample adds to each component an integer of at most 2^15 in magnitude, so
+// while a float sum stays within 2^24 every one of its additions is exact, and
+// any exact arithmetic gives the same value.
+//  * Exact phase: chunks of 64 samples through the dp4a tile loop, into int32
+//    sums that start from the buffer's.  Before a chunk the block checks that
+//    none of its sums can leave [-2^24, 2^24] within it.
+//  * Float phase, from the first chunk for which that check fails on: the
+//    samples' exact product sums added one by one, in time order, with one
+//    rounding each.
+// Gaussian samples of sigma 16 stay in the exact phase for 32000 samples (an
+// autocorrelation adds 512 a sample; the blocks off the diagonal stay much
+// longer).  dp4a does 4 samples' products for two issue slots of the pipe that
+// takes 4 x 3 float operations otherwise: N=64, F=10, T=1024 from 117 us per
+// call to 42 us, N=256 from 353 us to 121 us.
+// Either phase forbids time splits; the small blocks balance the SMs.
+constexpr int kTcF = 32;                         // samples per chunk of the float phase
 constexpr int kRawPanelF = kTcF * kRowBytes;     // 4 KiB
 constexpr int kFloatPanel = kTcF * kBlk;         // float4 entries: [sample][slot]
 constexpr int kFloatPanelRows = kTcF * kRows;    // the row block's 16 stations
+constexpr int kExactLimit = 1 << 24;             // float sums up to here are exact
+constexpr int kExactChunk = kTcD << 15;          // most that a chunk adds to a sum
 
 __device__ __forceinline__ void to_floats(const uint8_t *raw, float4 *fl) {
   for (int u = threadIdx.x; u < kTcF * kBlk; u += kThreads) {
@@ -321,112 +348,203 @@ __device__ __forceinline__ void to_floats_rows(const uint8_t *raw, float4 *fl) {
   }
 }
 
-// Dynamic shared memory of the FP32 kernel: raw panels [2 buffers][row,
-// column], the converted row and column panels, two mbarriers, and room to
-// align the panels to 128 bytes.
-constexpr int kSmemFp32 =
-    2 * 2 * kRawPanelF + (kFloatPanelRows + kFloatPanel) * 16 + 16 + 128;
-// five CTAs per SM by shared memory (80 registers a thread would allow six)
+// Dynamic shared memory of the FP32 kernel: the dp4a kernel's panels and words,
+// or the float phase's raw panels [2 buffers][row, column] and converted row
+// and column panels in the same place; then four mbarriers (two a phase), and
+// room to align the panels to 128 bytes.
+constexpr int kPanelsFp32 = 2 * 2 * kRawPanel + kWordPanelRows + kWordPanel;
+constexpr int kSmemFp32 = kPanelsFp32 + 32 + 128;
+static_assert(2 * 2 * kRawPanelF + (kFloatPanelRows + kFloatPanel) * 16 <= kPanelsFp32,
+              "the float phase's panels take the exact phase's place");
 static_assert(5 * (kSmemFp32 + 1024) <= 228 * 1024, "five FP32 CTAs per SM");
 
-__global__ void __launch_bounds__(kThreads) xengine_fp32_kernel(const __grid_constant__ Params p) {
+// i1 - i2 where only the difference is known to fit 32 bits (each half may have
+// wrapped).
+__device__ __forceinline__ int difference(int i1, int i2) { return (int)((unsigned)i1 - (unsigned)i2); }
+
+// The thread's tile in the buffer: baseline (i, j) of its 2x2 stations, and
+// whether the tile position holds one.
+__device__ __forceinline__ float4 *float_slot(const Params &p, int f, int i, int j) {
+  return (float4 *)((float *)p.state +
+                    ((long long)f * p.nbaseline + (long long)i * (i + 1) / 2 + j) * 8);
+}
+
+__global__ void __launch_bounds__(kThreads, 5) xengine_fp32_kernel(const __grid_constant__ Params p) {
   extern __shared__ __align__(128) uint8_t dsm_raw[];
   uint8_t *dsm = (uint8_t *)(((uintptr_t)dsm_raw + 127) & ~(uintptr_t)127);
-  auto raw = (uint8_t(*)[2][kRawPanelF])dsm;
-  float4 *flr = (float4 *)(dsm + 2 * 2 * kRawPanelF);   // row panel, 16 slots
-  float4 *flc = flr + kFloatPanelRows;                   // column panel, 32 slots
-  uint64_t *bars = (uint64_t *)(flc + kFloatPanel);
+  uint64_t *bars = (uint64_t *)(dsm + kPanelsFp32);
 
   const int f = p.f0 + (int)blockIdx.y;
   int rb, cb;   // row block of 16 stations, column block of 32
   decode_block(blockIdx.x, rb, cb);
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // ty 0..7
-  const int nchunks = (p.tcount + kTcF - 1) / kTcF;
-
-  // The accumulators continue the integration buffer's sums (0 after a
-  // clear), so an integration over several calls is one sum in time order.
-  float sr[2][2][2][2], si[2][2][2][2];
-  float *state = (float *)p.state;
-#pragma unroll
-  for (int rs = 0; rs < 2; ++rs)
-#pragma unroll
-    for (int cs = 0; cs < 2; ++cs) {
-      const int i = rb * kRows + 2 * ty + rs, j = cb * kBlk + 2 * tx + cs;
-      const bool mine = !p.overwrite && i < p.n && j <= i;
-      const float4 *src = (const float4 *)(state + ((long long)f * p.nbaseline +
-                                                    (long long)i * (i + 1) / 2 + j) * 8);
-#pragma unroll
-      for (int p1 = 0; p1 < 2; ++p1) {
-        const float4 o = mine ? src[p1] : make_float4(0.f, 0.f, 0.f, 0.f);
-        sr[rs][cs][p1][0] = o.x;
-        si[rs][cs][p1][0] = o.y;
-        sr[rs][cs][p1][1] = o.z;
-        si[rs][cs][p1][1] = o.w;
-      }
-    }
+  const int i0 = rb * kRows + 2 * ty, j0 = cb * kBlk + 2 * tx;
 
   const uint32_t bar0 = tc::smem_u32(&bars[0]);
+  auto raw = (uint8_t(*)[2][kRawPanel])dsm;
   if (threadIdx.x == 0) {
     asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&p.map) : "memory");
-    tc::mbar_init(bar0, 1);
-    tc::mbar_init(bar0 + 8, 1);
+    for (int q = 0; q < 4; ++q) tc::mbar_init(bar0 + 8 * q, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    issue_panels<kTcF>(raw[0], bar0, p, f, rb, cb, p.t0);
+    issue_panels<kTcD>(raw[0], bar0, p, p.map, f, rb, cb, p.t0);
   }
   __syncthreads();
 
-  for (int ch = 0; ch < nchunks; ++ch) {
-    const int buf = ch & 1;
-    // Chunk ch+1 goes into the other buffer, free since the end of chunk ch-1.
-    if (threadIdx.x == 0 && ch + 1 < nchunks)
-      issue_panels<kTcF>(raw[buf ^ 1], bar0 + 8 * (buf ^ 1), p, f, rb, cb, p.t0 + (ch + 1) * kTcF);
-    const bool got = tc::mbar_wait(bar0 + 8 * buf, (ch >> 1) & 1, nullptr);
-    if (__syncthreads_or(!got)) {
-      panel_timeout(p, bar0 + 8 * (buf ^ 1), ((ch + 1) >> 1) & 1, ch + 1 < nchunks);
-      return;
+  float sr[2][2][2][2], si[2][2][2][2];
+  int ch = 0;
+  {
+    // ---- exact phase
+    int4 *wrow = (int4 *)(dsm + 2 * 2 * kRawPanel);   // row words, 16 slots
+    int4 *wcol = wrow + kGroups * kRows;               // column words, 32 slots
+    const int nchunks = (p.tcount + kTcD - 1) / kTcD;
+    int re[2][2][2][2], i1[2][2][2][2], i2[2][2][2][2];
+    // The sums continue the buffer's (0 after a clear), so an integration over
+    // several calls is one sum in time order.  Sums past 2^24 do not fit the
+    // check below: top keeps it from passing, and the float phase reads them
+    // again.
+    int top = 0;
+#pragma unroll
+    for (int rs = 0; rs < 2; ++rs)
+#pragma unroll
+      for (int cs = 0; cs < 2; ++cs) {
+        const bool mine = !p.overwrite && i0 + rs < p.n && j0 + cs <= i0 + rs;
+        const float4 *src = float_slot(p, f, i0 + rs, j0 + cs);
+#pragma unroll
+        for (int p1 = 0; p1 < 2; ++p1) {
+          const float4 o = mine ? src[p1] : make_float4(0.f, 0.f, 0.f, 0.f);
+          const float big = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(o.w)));
+          if (!(big <= (float)kExactLimit)) top = kExactLimit;
+          re[rs][cs][p1][0] = (int)o.x;
+          i1[rs][cs][p1][0] = (int)o.y;
+          re[rs][cs][p1][1] = (int)o.z;
+          i1[rs][cs][p1][1] = (int)o.w;
+          i2[rs][cs][p1][0] = i2[rs][cs][p1][1] = 0;
+        }
+      }
+    int budget = 0;   // chunks that the last check covers
+    for (; ch < nchunks; ++ch) {
+      const int buf = ch & 1;
+      if (budget == 0) {
+        int m = top;
+#pragma unroll
+        for (int a = 0; a < 16; ++a)
+          m = max(m, max(abs((&re[0][0][0][0])[a]),
+                         abs(difference((&i1[0][0][0][0])[a], (&i2[0][0][0][0])[a]))));
+        if (!__syncthreads_or(m > kExactLimit - 4 * kExactChunk)) budget = 4;
+        else if (!__syncthreads_or(m > kExactLimit - kExactChunk)) budget = 1;
+        else break;
+      }
+      --budget;
+      // Chunk ch+1 goes into the other buffer, free since the end of chunk ch-1.
+      if (threadIdx.x == 0 && ch + 1 < nchunks)
+        issue_panels<kTcD>(raw[buf ^ 1], bar0 + 8 * (buf ^ 1), p, p.map, f, rb, cb,
+                           p.t0 + (ch + 1) * kTcD);
+      const bool got = tc::mbar_wait(bar0 + 8 * buf, (ch >> 1) & 1, nullptr);
+      if (__syncthreads_or(!got)) {
+        panel_timeout(p, bar0 + 8 * (buf ^ 1), ((ch + 1) >> 1) & 1, ch + 1 < nchunks);
+        return;
+      }
+      to_words<kRows>(raw[buf][0], wrow);
+      to_words<kBlk>(raw[buf][1], wcol);
+      __syncthreads();
+      dp4a_chunk(wrow, wcol, ty, tx, re, i1, i2);
+      __syncthreads();
     }
-    to_floats_rows(raw[buf][0], flr);
-    to_floats(raw[buf][1], flc);
-    __syncthreads();
-#pragma unroll 4
-    for (int t = 0; t < kTcF; ++t) {
-      float4 r[2], c[2];
-      r[0] = flr[t * kRows + ty];
-      r[1] = flr[t * kRows + 8 + ty];
-      c[0] = flc[t * kBlk + tx];
-      c[1] = flc[t * kBlk + 16 + tx];
+    if (ch < nchunks) {
+      // chunk ch, already on its way, lands before its place is used again
+      const bool got = tc::mbar_wait(bar0 + 8 * (ch & 1), (ch >> 1) & 1, nullptr);
+      if (__syncthreads_or(!got)) {
+        panel_timeout(p, 0, 0, false);
+        return;
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 16; ++a) {
+      (&sr[0][0][0][0])[a] = (float)(&re[0][0][0][0])[a];
+      (&si[0][0][0][0])[a] = (float)difference((&i1[0][0][0][0])[a], (&i2[0][0][0][0])[a]);
+    }
+  }
+
+  const int tdone = ch * kTcD;   // samples in the sums
+  if (tdone < p.tcount) {
+    // ---- float phase
+    auto rawf = (uint8_t(*)[2][kRawPanelF])dsm;
+    float4 *flr = (float4 *)(dsm + 2 * 2 * kRawPanelF);   // row panel, 16 slots
+    float4 *flc = flr + kFloatPanelRows;                   // column panel, 32 slots
+    const int tbeg = p.t0 + tdone;
+    const int nchunks = (p.tcount - tdone + kTcF - 1) / kTcF;
+    const uint32_t barf = bar0 + 16;
+    if (threadIdx.x == 0) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      issue_panels<kTcF>(rawf[0], barf, p, p.map_float, f, rb, cb, tbeg);
+    }
+    if (ch == 0) {
 #pragma unroll
       for (int rs = 0; rs < 2; ++rs)
 #pragma unroll
         for (int cs = 0; cs < 2; ++cs) {
-          const float ar[2] = {r[rs].x, r[rs].z}, ai[2] = {r[rs].y, r[rs].w};
-          const float br[2] = {c[cs].x, c[cs].z}, bi[2] = {c[cs].y, c[cs].w};
-          // xGPU's float arithmetic (omp_xengine.c:24-28): a sample's
-          // two products are summed first -- exactly: products of int8
-          // values and their sums are integers below 2^24 -- and the sum is
-          // added to the accumulator with one rounding.
+          const bool mine = !p.overwrite && i0 + rs < p.n && j0 + cs <= i0 + rs;
+          const float4 *src = float_slot(p, f, i0 + rs, j0 + cs);
 #pragma unroll
-          for (int p1 = 0; p1 < 2; ++p1)
-#pragma unroll
-            for (int p2 = 0; p2 < 2; ++p2) {
-              float &x = sr[rs][cs][p1][p2];
-              float &y = si[rs][cs][p1][p2];
-              x = __fadd_rn(x, __fmaf_rn(ai[p1], bi[p2], __fmul_rn(ar[p1], br[p2])));
-              y = __fadd_rn(y, __fmaf_rn(ai[p1], br[p2], -__fmul_rn(ar[p1], bi[p2])));
-            }
+          for (int p1 = 0; p1 < 2; ++p1) {
+            const float4 o = mine ? src[p1] : make_float4(0.f, 0.f, 0.f, 0.f);
+            sr[rs][cs][p1][0] = o.x;
+            si[rs][cs][p1][0] = o.y;
+            sr[rs][cs][p1][1] = o.z;
+            si[rs][cs][p1][1] = o.w;
+          }
         }
     }
-    __syncthreads();
+    for (int cf = 0; cf < nchunks; ++cf) {
+      const int buf = cf & 1;
+      if (threadIdx.x == 0 && cf + 1 < nchunks)
+        issue_panels<kTcF>(rawf[buf ^ 1], barf + 8 * (buf ^ 1), p, p.map_float, f, rb, cb,
+                           tbeg + (cf + 1) * kTcF);
+      const bool got = tc::mbar_wait(barf + 8 * buf, (cf >> 1) & 1, nullptr);
+      if (__syncthreads_or(!got)) {
+        panel_timeout(p, barf + 8 * (buf ^ 1), ((cf + 1) >> 1) & 1, cf + 1 < nchunks);
+        return;
+      }
+      to_floats_rows(rawf[buf][0], flr);
+      to_floats(rawf[buf][1], flc);
+      __syncthreads();
+#pragma unroll 4
+      for (int t = 0; t < kTcF; ++t) {
+        float4 r[2], c[2];
+        r[0] = flr[t * kRows + ty];
+        r[1] = flr[t * kRows + 8 + ty];
+        c[0] = flc[t * kBlk + tx];
+        c[1] = flc[t * kBlk + 16 + tx];
+#pragma unroll
+        for (int rs = 0; rs < 2; ++rs)
+#pragma unroll
+          for (int cs = 0; cs < 2; ++cs) {
+            const float ar[2] = {r[rs].x, r[rs].z}, ai[2] = {r[rs].y, r[rs].w};
+            const float br[2] = {c[cs].x, c[cs].z}, bi[2] = {c[cs].y, c[cs].w};
+            // A sample's two products are summed first -- exactly: products of
+            // int8 values and their sums are integers below 2^24 -- and the sum
+            // is added to the accumulator with one rounding.
+#pragma unroll
+            for (int p1 = 0; p1 < 2; ++p1)
+#pragma unroll
+              for (int p2 = 0; p2 < 2; ++p2) {
+                float &x = sr[rs][cs][p1][p2];
+                float &y = si[rs][cs][p1][p2];
+                x = __fadd_rn(x, __fmaf_rn(ai[p1], bi[p2], __fmul_rn(ar[p1], br[p2])));
+                y = __fadd_rn(y, __fmaf_rn(ai[p1], br[p2], -__fmul_rn(ar[p1], bi[p2])));
+              }
+          }
+      }
+      __syncthreads();
+    }
   }
 
 #pragma unroll
   for (int rs = 0; rs < 2; ++rs)
 #pragma unroll
     for (int cs = 0; cs < 2; ++cs) {
-      const int i = rb * kRows + 2 * ty + rs, j = cb * kBlk + 2 * tx + cs;
-      if (i >= p.n || j > i) continue;
-      float4 *dst = (float4 *)(state + ((long long)f * p.nbaseline +
-                                        (long long)i * (i + 1) / 2 + j) * 8);
+      if (i0 + rs >= p.n || j0 + cs > i0 + rs) continue;
+      float4 *dst = float_slot(p, f, i0 + rs, j0 + cs);
 #pragma unroll
       for (int p1 = 0; p1 < 2; ++p1)
         dst[p1] = make_float4(sr[rs][cs][p1][0], si[rs][cs][p1][0], sr[rs][cs][p1][1],
@@ -462,7 +580,7 @@ static int plain_splits(const Sizes &s, int fcount, int tcount, bool overlap) {
   return k < 1 ? 1 : (int)k;
 }
 
-// The kernels' dynamic shared memory (45.2 and 41.1 KB), allowed once per
+// The kernels' dynamic shared memory (45.2 KB each), allowed once per
 // device.
 static cudaError_t plain_configure_device() {
   static std::atomic<unsigned long long> done{0};
@@ -481,9 +599,8 @@ static cudaError_t plain_configure_device() {
 }
 
 static int plain_params(plain::Params *p, const int8_t *in, const Sizes &s, int t0, int tcount,
-                        void *state, int overwrite, int per, int rows, int *err, int stall,
-                        int f0) {
-  if (make_panel_map(&p->map, in, s, rows) != 0) return -1;
+                        void *state, int overwrite, int per, int *err, int stall, int f0) {
+  if (make_panel_map(&p->map, in, s, plain::kTcD) != 0) return -1;
   p->n = s.n;
   p->f = s.f;
   p->t0 = t0;
@@ -518,7 +635,7 @@ cudaError_t launch_plain_dp4a(const int8_t *in, const Sizes &s, int t0, int tcou
   cudaError_t e = plain_configure_device();
   if (e != cudaSuccess) return e;
   plain::Params p;
-  if (plain_params(&p, in, s, t0, tcount, state, overwrite, per, plain::kTcD, err, stall, f0) != 0)
+  if (plain_params(&p, in, s, t0, tcount, state, overwrite, per, err, stall, f0) != 0)
     return cudaErrorInvalidValue;
   p.overlap = (overlap && !overwrite) ? 1 : 0;
   // Programmatic launch: the grid may start beside the previous kernel's last
@@ -544,8 +661,8 @@ cudaError_t launch_plain_fp32(const int8_t *in, const Sizes &s, int t0, int tcou
   cudaError_t e = plain_configure_device();
   if (e != cudaSuccess) return e;
   plain::Params p;
-  if (plain_params(&p, in, s, t0, tcount, state, overwrite, tcount, plain::kTcF, err, stall,
-                   f0) != 0)
+  if (plain_params(&p, in, s, t0, tcount, state, overwrite, tcount, err, stall, f0) != 0 ||
+      make_panel_map(&p.map_float, in, s, plain::kTcF) != 0)
     return cudaErrorInvalidValue;
   plain::xengine_fp32_kernel<<<plain_grid(s, fcount), plain::kThreads, plain::kSmemFp32,
                                st>>>(p);
