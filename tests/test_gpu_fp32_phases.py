@@ -1,8 +1,9 @@
 """The FP32 engine's two phases (integer arithmetic while every float sum is
 exact, float arithmetic from there on) give the bits of xGPU's float engine:
 integrations that stay exact, that leave the exact phase in the first chunk, in
-a later one, at the check that covers four chunks or one, and calls that start
-from sums already past 2^24.  The oracle's float engine restates
+a later one, at the check that covers four chunks or one, calls that start
+from sums already past 2^24, and launches of every number of time pieces (one
+to eight: 256 stations x 6 channels and more than 32768 samples run whole).  The oracle's float engine restates
 omp_xengine.c:24-28 term for term, so the tolerance is zero."""
 import numpy as np
 import pytest
@@ -27,7 +28,8 @@ def samples(kind, n, f, t, rng):
 
 @pytest.mark.parametrize("kind", ["gauss", "full", "mixed", "late"])
 @pytest.mark.parametrize("n,f,t,calls", [(16, 1, 64, 1), (48, 2, 448, 1), (32, 1, 512, 2),
-                                         (64, 2, 1040, 3), (80, 1, 2064, 2), (32, 10, 6400, 1)])
+                                         (64, 2, 1040, 3), (80, 1, 2064, 2), (32, 10, 6400, 1),
+                                         (256, 6, 192, 3), (128, 13, 528, 2), (16, 1, 33024, 1)])
 def test_phases_equal_the_float_engine(xg, oracle_mod, kind, n, f, t, calls):
     rng = np.random.default_rng(n * 7919 + t)
     xs = [samples(kind, n, f, t, rng).reshape(-1) for _ in range(calls)]

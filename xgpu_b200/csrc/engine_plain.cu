@@ -123,9 +123,11 @@ __device__ __forceinline__ int dp4a(int a, int b, int c) {
 }
 
 // raw [sample][station][4 bytes] -> words [group][slot][4 words of 4 samples]
-// for the `slots` stations of a panel (32, or the row panel's first 16).
+// for the `slots` stations of a panel (32, or the row panel's first 16).  power:
+// adds the power of the two inputs of the station in the thread's slot
+// (threadIdx.x % kSlots for every item of a thread).
 template <int kSlots>
-__device__ __forceinline__ void to_words(const uint8_t *raw, int4 *words) {
+__device__ __forceinline__ void to_words(const uint8_t *raw, int4 *words, int *power = nullptr) {
   for (int u = threadIdx.x; u < kGroups * kSlots; u += kThreads) {
     const int g = u / kSlots, q = u % kSlots;
     const int s = kSlots == kBlk ? station_of_slot(q) : row_station_of_slot(q);
@@ -140,6 +142,10 @@ __device__ __forceinline__ void to_words(const uint8_t *raw, int4 *words) {
     o.z = (int)__byte_perm(hi01, hi23, 0x5410);  // Y re
     o.w = (int)__byte_perm(hi01, hi23, 0x7632);  // Y im
     words[g * kSlots + q] = o;
+    if (power) {
+      power[0] = dp4a(o.x, o.x, dp4a(o.y, o.y, power[0]));
+      power[1] = dp4a(o.z, o.z, dp4a(o.w, o.w, power[1]));
+    }
   }
 }
 
@@ -322,8 +328,10 @@ __global__ void __launch_bounds__(kThreads, 5) xengine_dp4a_kernel(const __grid_
 // autocorrelation adds 512 a sample; the blocks off the diagonal stay much
 // longer).  dp4a does 4 samples' products for two issue slots of the pipe that
 // takes 4 x 3 float operations otherwise: N=64, F=10, T=1024 from 117 us per
-// call to 42 us, N=256 from 353 us to 121 us.
-// Either phase forbids time splits; the small blocks balance the SMs.
+// call to 42 us, N=256 from 353 us to 125 us.  The float phase works on both
+// column polarisations at once with packed float pairs: the float pipe's rate
+// is the same, but half the instructions leave issue slots for the operand
+// loads (sums past 2^24 throughout, N=64: 113 to 98 us; N=256: 354 to 288).
 constexpr int kTcF = 32;                         // samples per chunk of the float phase
 constexpr int kRawPanelF = kTcF * kRowBytes;     // 4 KiB
 constexpr int kFloatPanel = kTcF * kBlk;         // float4 entries: [sample][slot]
@@ -331,15 +339,47 @@ constexpr int kFloatPanelRows = kTcF * kRows;    // the row block's 16 stations
 constexpr int kExactLimit = 1 << 24;             // float sums up to here are exact
 constexpr int kExactChunk = kTcD << 15;          // most that a chunk adds to a sum
 
+// Two floats in one register pair: sm_100's packed float instructions round
+// each half as the scalar ones do.
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair(float a, float b) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 halves(f32x2 v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+
+// raw [sample][station][4 bytes] -> [sample][slot] {X re, Y re, X im, Y im}: the
+// two column polarisations of each part side by side.
 __device__ __forceinline__ void to_floats(const uint8_t *raw, float4 *fl) {
   for (int u = threadIdx.x; u < kTcF * kBlk; u += kThreads) {
     const int t = u / kBlk, q = u % kBlk, s = station_of_slot(q);
     const char4 b = *(const char4 *)(raw + t * kRowBytes + s * 4);
-    fl[t * kBlk + q] = make_float4((float)b.x, (float)b.y, (float)b.z, (float)b.w);
+    fl[t * kBlk + q] = make_float4((float)b.x, (float)b.z, (float)b.y, (float)b.w);
   }
 }
 
-// The row panel: the first 16 stations of a 32-station panel.
+// The row panel, {X re, X im, Y re, Y im}: the first 16 stations of a 32-station
+// panel.
 __device__ __forceinline__ void to_floats_rows(const uint8_t *raw, float4 *fl) {
   for (int u = threadIdx.x; u < kTcF * kRows; u += kThreads) {
     const int t = u / kRows, q = u % kRows, s = row_station_of_slot(q);
@@ -350,50 +390,137 @@ __device__ __forceinline__ void to_floats_rows(const uint8_t *raw, float4 *fl) {
 
 // Dynamic shared memory of the FP32 kernel: the dp4a kernel's panels and words,
 // or the float phase's raw panels [2 buffers][row, column] and converted row
-// and column panels in the same place; then four mbarriers (two a phase), and
-// room to align the panels to 128 bytes.
+// and column panels in the same place; then four mbarriers (two a phase), what
+// the CTAs of a split call tell one another, and room to align the panels to
+// 128 bytes.
 constexpr int kPanelsFp32 = 2 * 2 * kRawPanel + kWordPanelRows + kWordPanel;
-constexpr int kSmemFp32 = kPanelsFp32 + 32 + 128;
+constexpr int kBarriersFp32 = 4;
 static_assert(2 * 2 * kRawPanelF + (kFloatPanelRows + kFloatPanel) * 16 <= kPanelsFp32,
               "the float phase's panels take the exact phase's place");
-static_assert(5 * (kSmemFp32 + 1024) <= 228 * 1024, "five FP32 CTAs per SM");
 
 // i1 - i2 where only the difference is known to fit 32 bits (each half may have
 // wrapped).
 __device__ __forceinline__ int difference(int i1, int i2) { return (int)((unsigned)i1 - (unsigned)i2); }
 
-// The thread's tile in the buffer: baseline (i, j) of its 2x2 stations, and
-// whether the tile position holds one.
-__device__ __forceinline__ float4 *float_slot(const Params &p, int f, int i, int j) {
-  return (float4 *)((float *)p.state +
-                    ((long long)f * p.nbaseline + (long long)i * (i + 1) / 2 + j) * 8);
+constexpr int kSmemFp32 = kPanelsFp32 + 8 * kBarriersFp32 + 40 + 128;
+static_assert(8 * kThreads * 16 <= 2 * 2 * kRawPanel, "the pieces' sums fit the panels");
+static_assert(5 * (kSmemFp32 + 128 + 1024) <= 228 * 1024, "five FP32 CTAs per SM");
+
+// The thread's 2x2 stations x 4 products as eight parts e = (rs, cs, p1) of
+// {re, im} x p2.  buffer_slot: part e of the tile at stations i0, j0.
+__device__ __forceinline__ float4 *buffer_slot(const Params &p, int f, int i0, int j0, int e) {
+  const long long i = i0 + (e >> 2), j = j0 + ((e >> 1) & 1);
+  return (float4 *)((float *)p.state + ((long long)f * p.nbaseline + i * (i + 1) / 2 + j) * 8) +
+         (e & 1);
 }
 
-__global__ void __launch_bounds__(kThreads, 5) xengine_fp32_kernel(const __grid_constant__ Params p) {
-  extern __shared__ __align__(128) uint8_t dsm_raw[];
-  uint8_t *dsm = (uint8_t *)(((uintptr_t)dsm_raw + 127) & ~(uintptr_t)127);
-  uint64_t *bars = (uint64_t *)(dsm + kPanelsFp32);
+// Whether the buffer has part e (a baseline of the array, on or below the
+// diagonal).
+__device__ __forceinline__ bool in_buffer(const Params &p, int i0, int j0, int e) {
+  const int i = i0 + (e >> 2), j = j0 + ((e >> 1) & 1);
+  return i < p.n && j <= i;
+}
 
-  const int f = p.f0 + (int)blockIdx.y;
-  int rb, cb;   // row block of 16 stations, column block of 32
-  decode_block(blockIdx.x, rb, cb);
+// The sums that the call continues: the buffer's, or zeros after a clear.
+__device__ __forceinline__ float4 buffer_part(const Params &p, int f, int i0, int j0, int e) {
+  return !p.overwrite && in_buffer(p, i0, j0, e) ? *buffer_slot(p, f, i0, j0, e)
+                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+}
+
+__device__ __forceinline__ float largest(float4 v) {
+  return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+}
+
+// The float phase: samples tbeg .. t0 + tcount - 1, one by one, into parts
+// e0 .. e0 + kParts - 1 (e0 a multiple of kParts).  barf: two initialised
+// mbarriers.  False: a panel never came (the error word is set).
+template <int kParts>
+__device__ __forceinline__ bool float_phase(const Params &p, uint8_t *dsm, uint32_t barf, int f,
+                                            int rb, int cb, int tbeg, int e0,
+                                            float4 (&sum)[kParts]) {
+  constexpr int kR = kParts == 8 ? 2 : 1;   // row stations, column stations and row
+  constexpr int kC = kParts >= 4 ? 2 : 1;   // polarisations among the parts
+  constexpr int kP = kParts >= 2 ? 2 : 1;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  auto raw = (uint8_t(*)[2][kRawPanelF])dsm;
+  float4 *flr = (float4 *)(dsm + 2 * 2 * kRawPanelF);   // row panel, 16 slots
+  float4 *flc = flr + kFloatPanelRows;                   // column panel, 32 slots
+  const float4 *row = flr + (kR == 2 ? 0 : e0 >> 2) * 8 + ty;
+  const float4 *col = flc + (kC == 2 ? 0 : (e0 >> 1) & 1) * 16 + tx;
+  const bool y = kP == 1 && (e0 & 1);
+  const int nchunks = (p.t0 + p.tcount - tbeg + kTcF - 1) / kTcF;
+  f32x2 xr[kParts], xi[kParts];   // real and imaginary sums of both column polarisations
+#pragma unroll
+  for (int k = 0; k < kParts; ++k) {
+    xr[k] = pair(sum[k].x, sum[k].z);
+    xi[k] = pair(sum[k].y, sum[k].w);
+  }
+  if (threadIdx.x == 0) {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    issue_panels<kTcF>(raw[0], barf, p, p.map_float, f, rb, cb, tbeg);
+  }
+  for (int ch = 0; ch < nchunks; ++ch) {
+    const int buf = ch & 1;
+    // Chunk ch+1 goes into the other buffer, free since the end of chunk ch-1.
+    if (threadIdx.x == 0 && ch + 1 < nchunks)
+      issue_panels<kTcF>(raw[buf ^ 1], barf + 8 * (buf ^ 1), p, p.map_float, f, rb, cb,
+                         tbeg + (ch + 1) * kTcF);
+    const bool got = tc::mbar_wait(barf + 8 * buf, (ch >> 1) & 1, nullptr);
+    if (__syncthreads_or(!got)) {
+      panel_timeout(p, barf + 8 * (buf ^ 1), ((ch + 1) >> 1) & 1, ch + 1 < nchunks);
+      return false;
+    }
+    to_floats_rows(raw[buf][0], flr);
+    to_floats(raw[buf][1], flc);
+    __syncthreads();
+#pragma unroll 4
+    for (int t = 0; t < kTcF; ++t) {
+      float4 r[kR];
+      f32x2 br[kC], bi[kC], nbi[kC];   // both polarisations of a column station, and -bi
+#pragma unroll
+      for (int q = 0; q < kR; ++q) r[q] = row[t * kRows + 8 * q];
+#pragma unroll
+      for (int q = 0; q < kC; ++q) {
+        const float4 c = col[t * kBlk + 16 * q];
+        br[q] = pair(c.x, c.y);
+        bi[q] = pair(c.z, c.w);
+        nbi[q] = pair(-c.z, -c.w);
+      }
+#pragma unroll
+      for (int k = 0; k < kParts; ++k) {
+        const int rs = k / (kC * kP), cs = k / kP % kC;
+        const bool p1 = kP == 2 ? k % 2 == 1 : y;
+        const float re = p1 ? r[rs].z : r[rs].x, im = p1 ? r[rs].w : r[rs].y;
+        const f32x2 ar = pair(re, re), ai = pair(im, im);
+        // A sample's two products are summed first -- exactly: products of
+        // int8 values and their sums are integers below 2^24 -- and the sum
+        // is added to the accumulator with one rounding.
+        xr[k] = add2(xr[k], fma2(ai, bi[cs], mul2(ar, br[cs])));
+        xi[k] = add2(xi[k], fma2(ai, br[cs], mul2(ar, nbi[cs])));
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int k = 0; k < kParts; ++k) {
+    const float2 re = halves(xr[k]), im = halves(xi[k]);
+    sum[k] = make_float4(re.x, im.x, re.y, im.y);
+  }
+  return true;
+}
+
+// The whole call by one CTA: the exact phase, then the float phase.  bar0:
+// four initialised mbarriers (two a phase).
+__device__ __forceinline__ void fp32_whole(const Params &p, uint8_t *dsm, uint32_t bar0, int f,
+                                           int rb, int cb) {
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;   // ty 0..7
   const int i0 = rb * kRows + 2 * ty, j0 = cb * kBlk + 2 * tx;
-
-  const uint32_t bar0 = tc::smem_u32(&bars[0]);
   auto raw = (uint8_t(*)[2][kRawPanel])dsm;
-  if (threadIdx.x == 0) {
-    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&p.map) : "memory");
-    for (int q = 0; q < 4; ++q) tc::mbar_init(bar0 + 8 * q, 1);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    issue_panels<kTcD>(raw[0], bar0, p, p.map, f, rb, cb, p.t0);
-  }
-  __syncthreads();
+  if (threadIdx.x == 0) issue_panels<kTcD>(raw[0], bar0, p, p.map, f, rb, cb, p.t0);
 
-  float sr[2][2][2][2], si[2][2][2][2];
+  float4 sum[8];
   int ch = 0;
   {
-    // ---- exact phase
     int4 *wrow = (int4 *)(dsm + 2 * 2 * kRawPanel);   // row words, 16 slots
     int4 *wcol = wrow + kGroups * kRows;               // column words, 32 slots
     const int nchunks = (p.tcount + kTcD - 1) / kTcD;
@@ -404,23 +531,16 @@ __global__ void __launch_bounds__(kThreads, 5) xengine_fp32_kernel(const __grid_
     // again.
     int top = 0;
 #pragma unroll
-    for (int rs = 0; rs < 2; ++rs)
-#pragma unroll
-      for (int cs = 0; cs < 2; ++cs) {
-        const bool mine = !p.overwrite && i0 + rs < p.n && j0 + cs <= i0 + rs;
-        const float4 *src = float_slot(p, f, i0 + rs, j0 + cs);
-#pragma unroll
-        for (int p1 = 0; p1 < 2; ++p1) {
-          const float4 o = mine ? src[p1] : make_float4(0.f, 0.f, 0.f, 0.f);
-          const float big = fmaxf(fmaxf(fabsf(o.x), fabsf(o.y)), fmaxf(fabsf(o.z), fabsf(o.w)));
-          if (!(big <= (float)kExactLimit)) top = kExactLimit;
-          re[rs][cs][p1][0] = (int)o.x;
-          i1[rs][cs][p1][0] = (int)o.y;
-          re[rs][cs][p1][1] = (int)o.z;
-          i1[rs][cs][p1][1] = (int)o.w;
-          i2[rs][cs][p1][0] = i2[rs][cs][p1][1] = 0;
-        }
-      }
+    for (int e = 0; e < 8; ++e) {
+      const int rs = e >> 2, cs = (e >> 1) & 1, p1 = e & 1;
+      const float4 o = buffer_part(p, f, i0, j0, e);
+      if (!(largest(o) <= (float)kExactLimit)) top = kExactLimit;
+      re[rs][cs][p1][0] = (int)o.x;
+      i1[rs][cs][p1][0] = (int)o.y;
+      re[rs][cs][p1][1] = (int)o.z;
+      i1[rs][cs][p1][1] = (int)o.w;
+      i2[rs][cs][p1][0] = i2[rs][cs][p1][1] = 0;
+    }
     int budget = 0;   // chunks that the last check covers
     for (; ch < nchunks; ++ch) {
       const int buf = ch & 1;
@@ -459,97 +579,226 @@ __global__ void __launch_bounds__(kThreads, 5) xengine_fp32_kernel(const __grid_
       }
     }
 #pragma unroll
-    for (int a = 0; a < 16; ++a) {
-      (&sr[0][0][0][0])[a] = (float)(&re[0][0][0][0])[a];
-      (&si[0][0][0][0])[a] = (float)difference((&i1[0][0][0][0])[a], (&i2[0][0][0][0])[a]);
+    for (int e = 0; e < 8; ++e) {
+      const int rs = e >> 2, cs = (e >> 1) & 1, p1 = e & 1;
+      sum[e] = make_float4((float)re[rs][cs][p1][0],
+                           (float)difference(i1[rs][cs][p1][0], i2[rs][cs][p1][0]),
+                           (float)re[rs][cs][p1][1],
+                           (float)difference(i1[rs][cs][p1][1], i2[rs][cs][p1][1]));
     }
   }
-
-  const int tdone = ch * kTcD;   // samples in the sums
-  if (tdone < p.tcount) {
-    // ---- float phase
-    auto rawf = (uint8_t(*)[2][kRawPanelF])dsm;
-    float4 *flr = (float4 *)(dsm + 2 * 2 * kRawPanelF);   // row panel, 16 slots
-    float4 *flc = flr + kFloatPanelRows;                   // column panel, 32 slots
-    const int tbeg = p.t0 + tdone;
-    const int nchunks = (p.tcount - tdone + kTcF - 1) / kTcF;
-    const uint32_t barf = bar0 + 16;
-    if (threadIdx.x == 0) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      issue_panels<kTcF>(rawf[0], barf, p, p.map_float, f, rb, cb, tbeg);
-    }
+  if (ch * kTcD < p.tcount) {
     if (ch == 0) {
 #pragma unroll
-      for (int rs = 0; rs < 2; ++rs)
-#pragma unroll
-        for (int cs = 0; cs < 2; ++cs) {
-          const bool mine = !p.overwrite && i0 + rs < p.n && j0 + cs <= i0 + rs;
-          const float4 *src = float_slot(p, f, i0 + rs, j0 + cs);
-#pragma unroll
-          for (int p1 = 0; p1 < 2; ++p1) {
-            const float4 o = mine ? src[p1] : make_float4(0.f, 0.f, 0.f, 0.f);
-            sr[rs][cs][p1][0] = o.x;
-            si[rs][cs][p1][0] = o.y;
-            sr[rs][cs][p1][1] = o.z;
-            si[rs][cs][p1][1] = o.w;
-          }
-        }
+      for (int e = 0; e < 8; ++e) sum[e] = buffer_part(p, f, i0, j0, e);
     }
-    for (int cf = 0; cf < nchunks; ++cf) {
-      const int buf = cf & 1;
-      if (threadIdx.x == 0 && cf + 1 < nchunks)
-        issue_panels<kTcF>(rawf[buf ^ 1], barf + 8 * (buf ^ 1), p, p.map_float, f, rb, cb,
-                           tbeg + (cf + 1) * kTcF);
-      const bool got = tc::mbar_wait(barf + 8 * buf, (cf >> 1) & 1, nullptr);
-      if (__syncthreads_or(!got)) {
-        panel_timeout(p, barf + 8 * (buf ^ 1), ((cf + 1) >> 1) & 1, cf + 1 < nchunks);
-        return;
-      }
-      to_floats_rows(rawf[buf][0], flr);
-      to_floats(rawf[buf][1], flc);
-      __syncthreads();
-#pragma unroll 4
-      for (int t = 0; t < kTcF; ++t) {
-        float4 r[2], c[2];
-        r[0] = flr[t * kRows + ty];
-        r[1] = flr[t * kRows + 8 + ty];
-        c[0] = flc[t * kBlk + tx];
-        c[1] = flc[t * kBlk + 16 + tx];
+    if (!float_phase<8>(p, dsm, bar0 + 16, f, rb, cb, p.t0 + ch * kTcD, 0, sum)) return;
+  }
 #pragma unroll
-        for (int rs = 0; rs < 2; ++rs)
+  for (int e = 0; e < 8; ++e)
+    if (in_buffer(p, i0, j0, e)) *buffer_slot(p, f, i0, j0, e) = sum[e];
+}
+
+// ---- the call split over a cluster
+// A launch with few blocks (small arrays, few channels) leaves SMs idle, and
+// alone on its SM a block takes 2.6 us per 64 samples where the dp4a pipe
+// needs 1.0.  So a cluster of kPieces CTAs shares the block:
+//  * first each takes a piece of the call's samples, with exact int32 sums
+//    from zero, and the pieces' sums are added through distributed shared
+//    memory.  That equals the sums in time order if no partial sum could have
+//    passed 2^24 anywhere in the call: within a piece each is at most |sum
+//    before the piece| + sum_t |x_i| |x_j| <= |sum before the piece| + the
+//    larger of the two inputs' powers in the piece (Cauchy-Schwarz).  The
+//    powers come from the converted words on the way, four dp4a an item;
+//  * when the buffer's sums are past 2^24 already (checked first), or the bound
+//    does not hold at the end, the float phase over all samples, each CTA
+//    keeping 8 / kPieces of the eight parts of every thread's tile.
+// Per call in chains at N=64, F=10, T=1024: 41.6 us whole, 20.0 in four pieces;
+// at N=16, F=1, T=512: 22 and 8; with samples of sigma 120, past 2^24 from the
+// second call on, at N=64: 98 and 95.
+struct SplitShared {
+  int past;            // CTAs whose share of the buffer is past 2^24, or breaks the bound
+  unsigned power[8];   // each piece's largest input power
+};
+static_assert(sizeof(SplitShared) <= 40, "room in the dynamic shared memory");
+constexpr int kFailed = 1 << 16;   // added to past by a CTA whose panels never came
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t in_cta(uint32_t local, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(local), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void add_in_cta(uint32_t local, uint32_t rank, unsigned v) {
+  asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(in_cta(local, rank)),
+               "r"(v)
+               : "memory");
+}
+__device__ __forceinline__ int4 ld_in_cta(uint32_t local, uint32_t rank) {
+  int4 v;
+  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "r"(in_cta(local, rank))
+               : "memory");
+  return v;
+}
+
+// bar0: four initialised mbarriers (two for the pieces, two for the float
+// phase).
+template <int kPieces>
+__device__ __forceinline__ void fp32_split(const Params &p, uint8_t *dsm, uint32_t bar0,
+                                           SplitShared *sh, int f, int rb, int cb) {
+  constexpr int kParts = 8 / kPieces;
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  const int i0 = rb * kRows + 2 * ty, j0 = cb * kBlk + 2 * tx;
+  const int z = (int)blockIdx.z;   // rank in the cluster
+  const int e0 = z * kParts;       // this CTA's share of the parts
+  const int tbeg = p.t0 + z * p.per, tend = min(p.t0 + p.tcount, tbeg + p.per);
+  const int nchunks = tbeg < tend ? (tend - tbeg + kTcD - 1) / kTcD : 0;
+  auto raw = (uint8_t(*)[2][kRawPanel])dsm;
+  int4 *wrow = (int4 *)(dsm + 2 * 2 * kRawPanel);
+  int4 *wcol = wrow + kGroups * kRows;
+  const uint32_t past = tc::smem_u32(&sh->past), power = tc::smem_u32(&sh->power[z]);
+
+  if (threadIdx.x == 0) {
+    sh->past = 0;
+    for (int q = 0; q < 8; ++q) sh->power[q] = 0;
+    if (nchunks) issue_panels<kTcD>(raw[0], bar0, p, p.map, f, rb, cb, tbeg);
+  }
+  bool big = false;
 #pragma unroll
-          for (int cs = 0; cs < 2; ++cs) {
-            const float ar[2] = {r[rs].x, r[rs].z}, ai[2] = {r[rs].y, r[rs].w};
-            const float br[2] = {c[cs].x, c[cs].z}, bi[2] = {c[cs].y, c[cs].w};
-            // A sample's two products are summed first -- exactly: products of
-            // int8 values and their sums are integers below 2^24 -- and the sum
-            // is added to the accumulator with one rounding.
+  for (int k = 0; k < kParts; ++k)
+    big |= !(largest(buffer_part(p, f, i0, j0, e0 + k)) <= (float)kExactLimit);
+  big = __syncthreads_or(big);
+  cluster_barrier();
+  if (big && threadIdx.x < kPieces) add_in_cta(past, threadIdx.x, 1);
+  cluster_barrier();
+  const bool skip = sh->past != 0;
+  bool ok = true;
+
+  int re[2][2][2][2], i1[2][2][2][2], i2[2][2][2][2];
 #pragma unroll
-            for (int p1 = 0; p1 < 2; ++p1)
+  for (int a = 0; a < 16; ++a) {
+    (&re[0][0][0][0])[a] = 0;
+    (&i1[0][0][0][0])[a] = 0;
+    (&i2[0][0][0][0])[a] = 0;
+  }
+  // powers of the two inputs of the row and of the column station in the slot
+  // that this thread converts (threadIdx.x % 16 and % 32)
+  int prow[2] = {0, 0}, pcol[2] = {0, 0};
+  const int todo = skip ? min(nchunks, 1) : nchunks;   // a skipped piece's first chunk still lands
+  for (int ch = 0; ch < todo; ++ch) {
+    const int buf = ch & 1;
+    if (threadIdx.x == 0 && ch + 1 < todo)
+      issue_panels<kTcD>(raw[buf ^ 1], bar0 + 8 * (buf ^ 1), p, p.map, f, rb, cb,
+                         tbeg + (ch + 1) * kTcD);
+    const bool got = tc::mbar_wait(bar0 + 8 * buf, (ch >> 1) & 1, nullptr);
+    if (__syncthreads_or(!got)) {
+      panel_timeout(p, bar0 + 8 * (buf ^ 1), ((ch + 1) >> 1) & 1, ch + 1 < todo);
+      ok = false;
+      break;
+    }
+    if (skip) break;
+    to_words<kRows>(raw[buf][0], wrow, prow);
+    to_words<kBlk>(raw[buf][1], wcol, pcol);
+    __syncthreads();
+    dp4a_chunk(wrow, wcol, ty, tx, re, i1, i2);
+    __syncthreads();
+  }
+  tc::pdl_trigger();
+  // The piece's sums into shared memory, part by part, 16 bytes a thread.
+  int4 *stage = (int4 *)dsm;
+  if (!skip) {
 #pragma unroll
-              for (int p2 = 0; p2 < 2; ++p2) {
-                float &x = sr[rs][cs][p1][p2];
-                float &y = si[rs][cs][p1][p2];
-                x = __fadd_rn(x, __fmaf_rn(ai[p1], bi[p2], __fmul_rn(ar[p1], br[p2])));
-                y = __fadd_rn(y, __fmaf_rn(ai[p1], br[p2], -__fmul_rn(ar[p1], bi[p2])));
-              }
-          }
-      }
-      __syncthreads();
+    for (int e = 0; e < 8; ++e) {
+      const int rs = e >> 2, cs = (e >> 1) & 1, p1 = e & 1;
+      stage[e * kThreads + threadIdx.x] =
+          make_int4(re[rs][cs][p1][0], difference(i1[rs][cs][p1][0], i2[rs][cs][p1][0]),
+                    re[rs][cs][p1][1], difference(i1[rs][cs][p1][1], i2[rs][cs][p1][1]));
+    }
+    // the powers of the block's row and column inputs, where the words were
+    unsigned *input = (unsigned *)wrow;
+    constexpr int kInputs = 2 * (kRows + kBlk);
+    if (threadIdx.x < kInputs) input[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int pol = 0; pol < 2; ++pol) {
+      atomicAdd(&input[2 * (threadIdx.x & 15) + pol], (unsigned)prow[pol]);
+      atomicAdd(&input[2 * (kRows + (threadIdx.x & 31)) + pol], (unsigned)pcol[pol]);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      unsigned m = 0;
+      for (int q = threadIdx.x; q < kInputs; q += 32) m = max(m, input[q]);
+      m = __reduce_max_sync(0xffffffffu, m);
+      if (threadIdx.x < kPieces) add_in_cta(power, threadIdx.x, m);
     }
   }
-
+  if (!ok && threadIdx.x < kPieces) add_in_cta(past, threadIdx.x, kFailed);
+  cluster_barrier();
+  float4 sum[kParts];
+  big = false;
+  if (!skip && ok) {
 #pragma unroll
-  for (int rs = 0; rs < 2; ++rs)
+    for (int k = 0; k < kParts; ++k) {
+      const float4 old = buffer_part(p, f, i0, j0, e0 + k);
+      int4 v = make_int4((int)old.x, (int)old.y, (int)old.z, (int)old.w);
 #pragma unroll
-    for (int cs = 0; cs < 2; ++cs) {
-      if (i0 + rs >= p.n || j0 + cs > i0 + rs) continue;
-      float4 *dst = float_slot(p, f, i0 + rs, j0 + cs);
-#pragma unroll
-      for (int p1 = 0; p1 < 2; ++p1)
-        dst[p1] = make_float4(sr[rs][cs][p1][0], si[rs][cs][p1][0], sr[rs][cs][p1][1],
-                              si[rs][cs][p1][1]);
+      for (int q = 0; q < kPieces; ++q) {
+        // the sums before piece q, within 2^24 as long as nothing was big
+        const int room = kExactLimit - (int)min(sh->power[q], 2u * kExactLimit);
+        big |= max(max(abs(v.x), abs(v.y)), max(abs(v.z), abs(v.w))) > room;
+        const int4 w = ld_in_cta(tc::smem_u32(&stage[(e0 + k) * kThreads + threadIdx.x]), q);
+        v.x += w.x;
+        v.y += w.y;
+        v.z += w.z;
+        v.w += w.w;
+      }
+      sum[k] = make_float4((float)v.x, (float)v.y, (float)v.z, (float)v.w);
     }
+  }
+  big = __syncthreads_or(big);
+  if (big && threadIdx.x < kPieces) add_in_cta(past, threadIdx.x, 1);
+  cluster_barrier();
+  if (sh->past >= kFailed) return;   // the error word is set
+  if (sh->past != 0) {
+#pragma unroll
+    for (int k = 0; k < kParts; ++k) sum[k] = buffer_part(p, f, i0, j0, e0 + k);
+    if (!float_phase<kParts>(p, dsm, bar0 + 16, f, rb, cb, p.t0, e0, sum)) return;
+  }
+#pragma unroll
+  for (int k = 0; k < kParts; ++k)
+    if (in_buffer(p, i0, j0, e0 + k)) *buffer_slot(p, f, i0, j0, e0 + k) = sum[k];
+}
+
+template <int kPieces>
+__global__ void __launch_bounds__(kThreads, 5) xengine_fp32_kernel(const __grid_constant__ Params p) {
+  extern __shared__ __align__(128) uint8_t dsm_raw[];
+  uint8_t *dsm = (uint8_t *)(((uintptr_t)dsm_raw + 127) & ~(uintptr_t)127);
+  const uint32_t bar0 = tc::smem_u32(dsm + kPanelsFp32);
+  const int f = p.f0 + (int)blockIdx.y;
+  int rb, cb;   // row block of 16 stations, column block of 32
+  decode_block(blockIdx.x, rb, cb);
+  if (threadIdx.x == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&p.map) : "memory");
+    for (int q = 0; q < kBarriersFp32; ++q) tc::mbar_init(bar0 + 8 * q, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncthreads();
+  // Programmatic launch: the prologue runs beside the previous kernel's end.  A
+  // grid that fills the SMs lets the next one in at once; a split one only when
+  // its sums are done, as CTAs that wait would unbalance the SMs for the grid
+  // after them (N=128 in two pieces: 64 against 45 us).
+  tc::pdl_wait();
+  if (kPieces == 1) tc::pdl_trigger();
+  if constexpr (kPieces > 1) {
+    fp32_split<kPieces>(p, dsm, bar0, (SplitShared *)(dsm + kPanelsFp32 + 8 * kBarriersFp32), f,
+                        rb, cb);
+  } else {
+    fp32_whole(p, dsm, bar0, f, rb, cb);
+  }
 }
 
 }  // namespace plain
@@ -580,6 +829,26 @@ static int plain_splits(const Sizes &s, int fcount, int tcount, bool overlap) {
   return k < 1 ? 1 : (int)k;
 }
 
+// Pieces of an FP32 launch (fp32_split), for 32768 samples at most (a piece's
+// power stays below 2^30).  Eight or four while the CTAs still fit the SMs about
+// once (5.5 each: N=128, F=10, 200 blocks, runs 44 us with four pieces, 60
+// without); a piece of fewer than 256 samples (eight) or 128 (four) costs more
+// in the exchange than it gains, unless the SMs are nearly empty.  Two pieces
+// only there: at 288 blocks they gain nothing (N=256, F=4: 60 against 60 us) and
+// the float phase loses 12%.
+static int fp32_pieces(const Sizes &s, int fcount, int tcount) {
+  const int sms = current_device_sms();
+  const dim3 g = plain_grid(s, fcount);
+  const long long blocks = (long long)g.x * g.y;
+  if (tcount > 32768) return 1;
+  for (int k = 8; k > 1; k /= 2) {
+    const bool sparse = blocks * k <= 2LL * sms;
+    const int least = k == 8 ? (sparse ? 64 : 256) : 128;
+    if ((sparse || (k > 2 && 2 * blocks * k <= 11LL * sms)) && tcount / k >= least) return k;
+  }
+  return 1;
+}
+
 // The kernels' dynamic shared memory (45.2 KB each), allowed once per
 // device.
 static cudaError_t plain_configure_device() {
@@ -591,9 +860,13 @@ static cudaError_t plain_configure_device() {
   if (bit && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
   e = cudaFuncSetAttribute(plain::xengine_dp4a_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            plain::kSmemDp4a);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(plain::xengine_fp32_kernel,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, plain::kSmemFp32);
+  const void *fp32[] = {(const void *)plain::xengine_fp32_kernel<1>,
+                        (const void *)plain::xengine_fp32_kernel<2>,
+                        (const void *)plain::xengine_fp32_kernel<4>,
+                        (const void *)plain::xengine_fp32_kernel<8>};
+  for (const void *k : fp32)
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, plain::kSmemFp32);
   if (e == cudaSuccess && bit) done.fetch_or(bit, std::memory_order_release);
   return e;
 }
@@ -660,13 +933,34 @@ cudaError_t launch_plain_fp32(const int8_t *in, const Sizes &s, int t0, int tcou
   if (f0 < 0 || fcount < 1 || f0 + fcount > s.f) return cudaErrorInvalidValue;
   cudaError_t e = plain_configure_device();
   if (e != cudaSuccess) return e;
+  const int pieces = fp32_pieces(s, fcount, tcount);
+  // samples per piece: a whole number of 64-sample chunks
+  int per = (tcount + pieces - 1) / pieces;
+  per = (per + plain::kTcD - 1) / plain::kTcD * plain::kTcD;
   plain::Params p;
-  if (plain_params(&p, in, s, t0, tcount, state, overwrite, tcount, err, stall, f0) != 0 ||
+  if (plain_params(&p, in, s, t0, tcount, state, overwrite, per, err, stall, f0) != 0 ||
       make_panel_map(&p.map_float, in, s, plain::kTcF) != 0)
     return cudaErrorInvalidValue;
-  plain::xengine_fp32_kernel<<<plain_grid(s, fcount), plain::kThreads, plain::kSmemFp32,
-                               st>>>(p);
-  return cudaGetLastError();
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = plain_grid(s, fcount, pieces);
+  cfg.blockDim = dim3(plain::kThreads);
+  cfg.dynamicSmemBytes = plain::kSmemFp32;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = (unsigned)pieces;
+  cfg.attrs = attr;
+  cfg.numAttrs = pieces > 1 ? 2 : 1;
+  switch (pieces) {
+    case 8: return cudaLaunchKernelEx(&cfg, plain::xengine_fp32_kernel<8>, p);
+    case 4: return cudaLaunchKernelEx(&cfg, plain::xengine_fp32_kernel<4>, p);
+    case 2: return cudaLaunchKernelEx(&cfg, plain::xengine_fp32_kernel<2>, p);
+    default: return cudaLaunchKernelEx(&cfg, plain::xengine_fp32_kernel<1>, p);
+  }
 }
 
 }  // namespace xgpu
