@@ -104,7 +104,7 @@ __device__ __forceinline__ void issue_panels(uint8_t (*raw)[NT * kRowBytes], uin
 __device__ __forceinline__ void panel_timeout(const Params &p, uint32_t other_bar,
                                               uint32_t other_parity, bool other_in_flight) {
   if (threadIdx.x == 0) {
-    if (p.err) atomicExch(p.err, kErrTimeoutPanel);
+    if (p.err) tc::report_error(p.err, kErrTimeoutPanel);
     if (other_in_flight && !p.stall) tc::mbar_wait(other_bar, other_parity, nullptr);
   }
 }

@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(kThreads, 1) xengine_tc_kernel(const __grid_co
   pdl_trigger();
 
   auto fail = [&](int code) {
-    atomicExch(p.err, code);
+    report_error(p.err, code);
     *abort_flag = 1;
   };
 

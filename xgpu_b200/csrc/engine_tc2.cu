@@ -387,7 +387,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPacked ? kThreadsPa
   pdl_trigger();
 
   auto fail = [&](int code) {
-    atomicExch(p.err, code);
+    report_error(p.err, code);
     *abort_flag = 1;
   };
 

@@ -2,8 +2,8 @@
 // input.
 //
 // Output orders (xgpu.h:45-47) are produced on the device from the triangular
-// integration buffer, so a dump copies exactly the requested layout to the
-// host.  The index maps follow the reference's writers and reorderers:
+// integration buffer, so a dump moves exactly the requested layout to the host.
+// The index maps follow the reference's writers and reorderers:
 //   TRIANGULAR_ORDER            kernel.cuh:96-117, cpu_util.c:161-162
 //   REAL_IMAG_TRIANGULAR_ORDER  kernel.cuh:72-95,  cpu_util.c:112-115
 //   REGISTER_TILE_...           kernel.cuh:49-71,  cpu_util.c:66-79
@@ -11,60 +11,151 @@
 
 #include "internal.h"
 #include "packed4.cuh"
+#include "tc_common.cuh"
 
 namespace xgpu {
 
 namespace fmt {
 
-struct Params {
-  const void *state;
-  int state_is_float;
-  int n, f;
-  long long nbaseline, mat_length;
-  int order, out_type;
-  uint32_t *out;  // matLength Complex = 2*matLength 32-bit words
-  long long u0, u1;   // the (channel, baseline, product) range formatted
-};
-
-__device__ __forceinline__ uint32_t convert(const void *state, int is_float, long long idx,
-                                            int out_type) {
-  if (is_float) {
-    const float v = ((const float *)state)[idx];
-    if (out_type == XGPU_INT32) return (uint32_t)__float2int_rn(v);
-    return __float_as_uint(v);
-  }
-  const long long v = ((const long long *)state)[idx];
+__device__ __forceinline__ uint32_t dump_word(long long v, int out_type) {
   if (out_type == XGPU_INT32) return (uint32_t)(unsigned long long)v;  // wraps like int32 sums
   return __float_as_uint(__ll2float_rn(v));
 }
 
-// One thread per (channel, baseline, polarisation product).
-__global__ void format_kernel(const Params p) {
-  for (long long u = p.u0 + blockIdx.x * (long long)blockDim.x + threadIdx.x; u < p.u1;
-       u += (long long)gridDim.x * blockDim.x) {
-    const int pp = (int)(u & 3);
-    const long long fk = u >> 2;
-    const int f = (int)(fk / p.nbaseline);
-    const long long k = fk - (long long)f * p.nbaseline;
-    const uint32_t re = convert(p.state, p.state_is_float, 2 * u, p.out_type);
-    const uint32_t im = convert(p.state, p.state_is_float, 2 * u + 1, p.out_type);
-    if (p.order == TRIANGULAR_ORDER) {
-      *(uint2 *)(p.out + 2 * u) = make_uint2(re, im);
-    } else if (p.order == REAL_IMAG_TRIANGULAR_ORDER) {
-      p.out[u] = re;
-      p.out[u + p.mat_length] = im;
+__device__ __forceinline__ uint32_t dump_word(float v, int out_type) {
+  if (out_type == XGPU_INT32) return (uint32_t)__float2int_rn(v);
+  return __float_as_uint(v);
+}
+
+// Register-tile order: baseline (i, j) in position k of a channel's slots, 2 x 2
+// planes of tiles (I, J) as rows of a triangle; j > i where a slot holds none.
+__device__ __forceinline__ void tile_slot(int k, int tiles, int &i, int &j) {
+  const int slot = k / tiles, q = k - slot * tiles;
+  int I = (int)((sqrtf(8.0f * (float)q + 1.0f) - 1.0f) * 0.5f);
+  while (I * (I + 1) / 2 > q) --I;
+  while ((I + 1) * (I + 2) / 2 <= q) ++I;
+  i = 2 * I + (slot & 1);
+  j = 2 * (q - I * (I + 1) / 2) + (slot >> 1);
+}
+
+// A dump into device memory: channel f0 + blockIdx.y, one thread per product,
+// striding over the channel in the order of the output (32-bit index arithmetic
+// within the channel); register-tile order's slots without a baseline get
+// zeros.  Programmatic: the launch latency passes under the previous kernel's
+// end.  Memory-bound: 16 (int64) or 8 (float) bytes in, 8 out.
+template <bool kFloat, bool kTiles>
+__global__ void __launch_bounds__(256) format_kernel(const void *state, int n, int nbaseline,
+                                                     int f0, const DumpOut o) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
+  const int f = f0 + (int)blockIdx.y;
+  const int tiles = (n / 2 + 1) * (n / 4);
+  const int words = 4 * (kTiles ? 4 * tiles : nbaseline);
+  const long long base = (long long)f * nbaseline * 4;
+  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < words; v += gridDim.x * blockDim.x) {
+    int u = v;   // product within the channel, triangular order
+    if (kTiles) {
+      int i, j;
+      tile_slot(v >> 2, tiles, i, j);
+      u = j <= i ? 4 * (i * (i + 1) / 2 + j) + (v & 3) : -1;
+    }
+    uint32_t re = 0, im = 0;
+    if (!kTiles || u >= 0) {
+      if (kFloat) {
+        const float2 x = ((const float2 *)state)[base + u];
+        re = dump_word(x.x, o.out_type);
+        im = dump_word(x.y, o.out_type);
+      } else {
+        const longlong2 x = ((const longlong2 *)state)[base + u];
+        re = dump_word(x.x, o.out_type);
+        im = dump_word(x.y, o.out_type);
+      }
+    }
+    if (!kTiles && o.order == TRIANGULAR_ORDER) {
+      *(uint2 *)(o.out + 2 * (base + v)) = make_uint2(re, im);
     } else {
-      int i = (int)((sqrt(8.0 * (double)k + 1.0) - 1.0) * 0.5);
-      while ((long long)i * (i + 1) / 2 > k) --i;
-      while ((long long)(i + 1) * (i + 2) / 2 <= k) ++i;
-      const int j = (int)(k - (long long)i * (i + 1) / 2);
-      const long long rtn = (long long)(p.n / 2 + 1) * (p.n / 4);
-      const int I = i >> 1, J = j >> 1, rx = i & 1, ry = j & 1;
-      const long long l =
-          (long long)f * 4 * rtn + (long long)(2 * ry + rx) * rtn + (long long)I * (I + 1) / 2 + J;
-      const long long w = l * 4 + pp;
-      p.out[w] = re;
-      p.out[w + p.mat_length] = im;
+      const long long w = (long long)f * words + v;
+      o.out[w] = re;
+      o.out[w + o.mat_length] = im;
+    }
+  }
+}
+
+// A dump into host memory that the device maps (16-byte aligned): 16 bytes of
+// the output per thread and step, a warp's 512 contiguous.  The host link sets
+// the pace: 10.5 MB take 209 us for any grid from 2048 threads on, 50 GB/s.
+// What the grid decides is how much waits for it: with the output's lines last
+// written by 16 processor cores, 75,000 threads still take 211 us, 2048 threads
+// 315 (and a copy engine, 190 us on untouched lines, 350).  Stores that wait
+// hold up every other SM's memory accesses meanwhile (a 256 MB read, 67 us
+// alone, took 248 beside them), so nothing is gained by running an engine launch
+// beside a dump.  Against one 8-byte store per product (16 blocks of 256 threads
+// per SM): dumps of 10.5, 16.9 and 6.5 MB 222 to 215, 346 to 338 and 145 to 139
+// us; a dumping call over host input (register-tile order, formatted in device
+// memory and copied before) 398 to 361 us.
+constexpr int kHostThreads = 128;
+constexpr int kHostBlocks = 4 * 148;
+constexpr long long kHostSmall = 512 << 10;   // bytes of output below which format_kernel's
+                                              // shorter code is through first (a call and a
+                                              // 33 KB dump: 22 us against 26)
+template <bool kFloat, bool kTiles>
+__global__ void __launch_bounds__(kHostThreads)
+    format_host_kernel(const void *state, int n, int nbaseline, int f0, int fcount,
+                       const DumpOut o) {
+  tc::pdl_wait();
+  tc::pdl_trigger();
+  constexpr int kSteps = 4;   // loads of four steps in flight per thread
+  const int tiles = (n / 2 + 1) * (n / 4);
+  const int slots = kTiles ? 4 * tiles : nbaseline;   // baselines' places per channel
+  const bool planes = kTiles || o.order != TRIANGULAR_ORDER;
+  const int each = planes ? 4 : 2;                    // products in 16 bytes
+  const long long first = (long long)f0 * slots * 4, total = (long long)fcount * slots * 4;
+  const long long stride = (long long)gridDim.x * kHostThreads;
+  // product `at` in triangular order: its two words
+  auto words = [&](long long at, uint32_t &re, uint32_t &im) {
+    if (kFloat) {
+      const float2 x = ((const float2 *)state)[at];
+      re = dump_word(x.x, o.out_type);
+      im = dump_word(x.y, o.out_type);
+    } else {
+      const longlong2 x = ((const longlong2 *)state)[at];
+      re = dump_word(x.x, o.out_type);
+      im = dump_word(x.y, o.out_type);
+    }
+  };
+  for (long long u0 = blockIdx.x * kHostThreads + threadIdx.x; u0 * each < total;
+       u0 += kSteps * stride) {
+    uint32_t re[kSteps][4], im[kSteps][4];
+#pragma unroll
+    for (int s = 0; s < kSteps; ++s) {
+      const long long v = (u0 + s * stride) * each;   // product's place in the output
+      if (v >= total) break;
+      long long at = first + v;
+      bool live = true;
+      if (kTiles) {
+        const int f = f0 + (int)((v >> 2) / slots), q = (int)((v >> 2) % slots);
+        int i, j;
+        tile_slot(q, tiles, i, j);
+        live = j <= i;
+        at = ((long long)f * nbaseline + i * (i + 1) / 2 + j) * 4;
+      }
+#pragma unroll
+      for (int pp = 0; pp < 4; ++pp) {
+        re[s][pp] = im[s][pp] = 0;
+        if (live && pp < each) words(at + pp, re[s][pp], im[s][pp]);
+      }
+    }
+#pragma unroll
+    for (int s = 0; s < kSteps; ++s) {
+      const long long v = (u0 + s * stride) * each;
+      if (v >= total) break;
+      uint32_t *d = o.out + (planes ? 1 : 2) * (first + v);
+      if (planes) {
+        *(uint4 *)d = make_uint4(re[s][0], re[s][1], re[s][2], re[s][3]);
+        *(uint4 *)(d + o.mat_length) = make_uint4(im[s][0], im[s][1], im[s][2], im[s][3]);
+      } else {
+        *(uint4 *)d = make_uint4(re[s][0], im[s][0], re[s][1], im[s][1]);
+      }
     }
   }
 }
@@ -183,26 +274,38 @@ static unsigned grid_for(long long work, int threads) {
 
 }  // namespace fmt
 
-cudaError_t launch_format(const void *state, int state_is_float, const Sizes &s, int order,
-                          int out_type, void *out, cudaStream_t st, int f0, int fcount) {
+cudaError_t launch_format(const void *state, int state_is_float, const Sizes &s, const DumpOut &o,
+                          cudaStream_t st, int f0, int fcount, bool host_out) {
   if (fcount < 0) fcount = s.f - f0;
   if (f0 < 0 || fcount < 1 || f0 + fcount > s.f) return cudaErrorInvalidValue;
-  if (order == REGISTER_TILE_TRIANGULAR_ORDER) {
-    // Slots that hold no baseline (kernel.cuh:65-71) stay zero: clear the
-    // channel range's words in both planes.
-    const long long per = s.mat_length / s.f;   // 32-bit words per channel and plane
-    for (int plane = 0; plane < 2; ++plane) {
-      cudaError_t e = cudaMemsetAsync((uint32_t *)out + plane * s.mat_length + f0 * per, 0,
-                                      (size_t)(fcount * per) * 4, st);
-      if (e != cudaSuccess) return e;
-    }
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const bool tiles = o.order == REGISTER_TILE_TRIANGULAR_ORDER;
+  if (host_out && ((uintptr_t)o.out & 15) == 0 &&
+      s.mat_length / s.f * fcount * 8 >= fmt::kHostSmall) {
+    const long long blocks =
+        (s.mat_length / s.f * fcount / 2 + fmt::kHostThreads - 1) / fmt::kHostThreads;
+    cfg.gridDim = dim3((unsigned)(blocks < fmt::kHostBlocks ? blocks : fmt::kHostBlocks));
+    cfg.blockDim = dim3(fmt::kHostThreads);
+    auto *k = state_is_float
+                  ? (tiles ? fmt::format_host_kernel<true, true> : fmt::format_host_kernel<true, false>)
+                  : (tiles ? fmt::format_host_kernel<false, true>
+                           : fmt::format_host_kernel<false, false>);
+    return cudaLaunchKernelEx(&cfg, k, state, s.n, (int)s.nbaseline, f0, fcount, o);
   }
-  const long long per_ch = s.nbaseline * 4;
-  fmt::Params p{state, state_is_float, s.n, s.f, s.nbaseline, s.mat_length, order, out_type,
-                (uint32_t *)out, f0 * per_ch, (f0 + fcount) * per_ch};
-  const long long work = fcount * per_ch;
-  fmt::format_kernel<<<fmt::grid_for(work, 256), 256, 0, st>>>(p);
-  return cudaGetLastError();
+  // about 16 blocks per SM in all, at least one per channel
+  const int blocks = (int)((s.mat_length / s.f + 255) / 256);
+  const int most = (148 * 16 + fcount - 1) / fcount;
+  cfg.gridDim = dim3((unsigned)(blocks < most ? blocks : most), (unsigned)fcount);
+  auto *k = state_is_float ? (tiles ? fmt::format_kernel<true, true> : fmt::format_kernel<true, false>)
+                           : (tiles ? fmt::format_kernel<false, true> : fmt::format_kernel<false, false>);
+  return cudaLaunchKernelEx(&cfg, k, state, s.n, (int)s.nbaseline, f0, o);
 }
 
 cudaError_t launch_unpack4(const uint8_t *in, int8_t *out, long long nsamples, cudaStream_t st) {

@@ -122,6 +122,12 @@ long long words_blocks(const Sizes &s);   // 32-station blocks per channel
 bool tc2_uses_words(int tcount, const TcTuning &tune);
 bool tc2_single_item(int tcount, const TcTuning &tune);
 long long words_elems(const Sizes &s);
+// A dump's destination: matLength Complex as 32-bit words.
+struct DumpOut {
+  uint32_t *out;
+  long long mat_length;
+  int order, out_type;
+};
 // overlap: the launch before it on `st` is an engine launch of the same
 // context (it may then start while that launch finishes).  store_state: the
 // int64 buffer holds nothing yet; the fold stores into it instead of adding.
@@ -167,12 +173,12 @@ cudaError_t tc2_set_smem_attribute();
 cudaError_t launch_unpack4(const uint8_t *in, int8_t *out, long long nsamples, cudaStream_t st);
 cudaError_t launch_unswizzle_dp4a(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st);
 cudaError_t launch_unblock32(const int8_t *in, int8_t *out, long long nbytes, cudaStream_t st);
-// state (int64 or float) -> Complex words in `order` of type out_type.
-// Channels [f0, f0 + fcount) of the buffer into `out` in the requested order
-// (fcount < 0: through the last channel); other channels' words are untouched.
-cudaError_t launch_format(const void *state, int state_is_float, const Sizes &s, int order,
-                          int out_type, void *out, cudaStream_t st, int f0 = 0,
-                          int fcount = -1);
+// Channels [f0, f0 + fcount) of the buffer (int64 or float) into o.out in its
+// order and type (fcount < 0: through the last channel; other channels' words
+// are untouched).  Launched programmatically.  host_out: the output is mapped
+// host memory.
+cudaError_t launch_format(const void *state, int state_is_float, const Sizes &s, const DumpOut &o,
+                          cudaStream_t st, int f0 = 0, int fcount = -1, bool host_out = false);
 cudaError_t launch_generate(void *out, size_t nbytes, int kind, unsigned long long seed,
                             double sigma, cudaStream_t st);
 

@@ -131,8 +131,9 @@ int correlate_static(const void *device_input, void *device_output, const XGPUCo
     if (launch_tc_tuned(map, s, t0, tc, state, t0 == 0 ? 1 : 0, err, st, tune, 0) != cudaSuccess)
       return XGPU_CUDA_ERROR;
   }
-  if (launch_format(state, 0, s, (int)c.matrix_order, (int)c.output_type, device_output, st) !=
-      cudaSuccess)
+  const DumpOut out{(uint32_t *)device_output, s.mat_length, (int)c.matrix_order,
+                    (int)c.output_type};
+  if (launch_format(state, 0, s, out, st) != cudaSuccess)
     return XGPU_CUDA_ERROR;
   int h_err = 0;
   if (cudaMemcpyAsync(&h_err, err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||

@@ -97,8 +97,10 @@ struct Internal {
   bool words_dirty = false;            // the words hold sums not yet in d_state
   bool words_stale = false;            // the words hold nothing, but are not zero
   void *d_out = nullptr;               // formatted dump
-  int *d_err = nullptr;                // device error word
-  int *h_err = nullptr;                // pinned copy of it
+  // Device error word: page-locked host memory that kernels write on a timeout
+  // (d_err is its device address) and the host reads after a wait, with no copy
+  // to queue and wait for.
+  int *h_err = nullptr, *d_err = nullptr;
 
   cudaStream_t s_copy = nullptr, s_comp = nullptr;
   cudaStream_t s_own = nullptr;  // the context's own compute stream
@@ -218,7 +220,6 @@ int free_device(Internal *in) {
   if (in->d_state) cudaFree(in->d_state);
   if (in->d_words) cudaFree(in->d_words);
   if (in->d_out) cudaFree(in->d_out);
-  if (in->d_err) cudaFree(in->d_err);
   if (in->h_err) cudaFreeHost(in->h_err);
   return XGPU_OK;
 }
@@ -441,19 +442,17 @@ int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool 
   return XGPU_OK;
 }
 
-// Read and clear the device error word.
-// Queued on `st` (default s_comp), which must be the stream whose completion
-// implies every engine launch's: the read and the wait are one round trip.
+// Wait for `st` (default s_comp; its completion must imply every engine
+// launch's), then read and clear the device error word.
 int check_device_error(Internal *in, cudaStream_t st = nullptr) {
   in->adding_tail = false;
-  if (!st) st = in->s_comp;
-  XGPU_CHECK(cudaMemcpyAsync(in->h_err, in->d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-  XGPU_CHECK(cudaStreamSynchronize(st));
-  if (*in->h_err != 0) {
+  XGPU_CHECK(cudaStreamSynchronize(st ? st : in->s_comp));
+  const int err = *(volatile int *)in->h_err;
+  if (err != 0) {
     fprintf(stderr, "xgpu: device wait timed out (code %d); results of this integration are invalid\n",
-            *in->h_err);
-    XGPU_CHECK(cudaMemsetAsync(in->d_err, 0, sizeof(int), in->s_comp));
+            err);
     XGPU_CHECK(cudaStreamSynchronize(in->s_comp));
+    *(volatile int *)in->h_err = 0;
     return XGPU_CUDA_ERROR;
   }
   return XGPU_OK;
@@ -461,18 +460,21 @@ int check_device_error(Internal *in, cudaStream_t st = nullptr) {
 
 // The device address of the caller's output (the host buffer at
 // output_offset) when the formatting kernel can store the dump straight into
-// it: triangular and real-imag orders, whose words the kernel writes in runs,
-// into page-locked memory the device maps, 8-byte aligned.  Those stores
-// cross the host link at the rate of a copy.  Otherwise nullptr: the dump is
-// formatted in device memory and copied.
-void *direct_output(XGPUContext *ctx, Internal *in) {
-  if (in->cfg.matrix_order == REGISTER_TILE_TRIANGULAR_ORDER) return nullptr;
+// it: page-locked memory that the device maps, 8-byte aligned.  Otherwise
+// nullptr: the dump is formatted in device memory and copied.
+void *direct_output(XGPUContext *ctx) {
   void *p = nullptr;
   if (cudaHostGetDevicePointer(&p, ctx->matrix_h + ctx->output_offset, 0) != cudaSuccess) {
     cudaGetLastError();
     return nullptr;
   }
   return ((uintptr_t)p & 7) == 0 ? p : nullptr;
+}
+
+// Where a dump's formatting writes: the caller's output, or d_out.
+DumpOut dump_out(const Internal *in, void *direct) {
+  return DumpOut{(uint32_t *)(direct ? direct : in->d_out), in->sz.mat_length,
+                 (int)in->cfg.matrix_order, (int)in->cfg.output_type};
 }
 
 int dump(XGPUContext *ctx, Internal *in) {
@@ -489,9 +491,9 @@ int dump(XGPUContext *ctx, Internal *in) {
     XGPU_CHECK(cudaMemsetAsync(in->d_state, 0, (size_t)in->sz.state_elems * (in->int_state ? 8 : 4),
                                in->s_comp));
   }
-  void *direct = direct_output(ctx, in);
-  XGPU_CHECK(launch_format(in->d_state, in->int_state ? 0 : 1, in->sz, in->cfg.matrix_order,
-                           in->cfg.output_type, direct ? direct : in->d_out, in->s_comp));
+  void *direct = direct_output(ctx);
+  XGPU_CHECK(launch_format(in->d_state, in->int_state ? 0 : 1, in->sz, dump_out(in, direct),
+                           in->s_comp, 0, -1, direct != nullptr));
   if (!direct)
     XGPU_CHECK(cudaMemcpyAsync(ctx->matrix_h + ctx->output_offset, in->d_out,
                                (size_t)in->sz.mat_length * sizeof(Complex),
@@ -576,9 +578,9 @@ int dump_call_grouped(XGPUContext *ctx, Internal *in, int b, int groups) {
   }
   XGPU_CHECK(cudaEventRecord(in->copy_done[b], in->s_copy));
   // Direct stores format on s_dump, beside the next group's engine; results
-  // formatted in device memory (register-tile order) format on s_comp and
-  // leave s_dump to the copies.
-  void *direct = direct_output(ctx, in);
+  // formatted in device memory (an output the device does not map) format on
+  // s_comp and leave s_dump to the copies.
+  void *direct = direct_output(ctx);
   cudaStream_t s_fmt = direct ? in->s_dump : in->s_comp;
   for (int k = 0; k < ng; ++k) {
     const int f0 = bound[k], fc = bound[k + 1] - bound[k];
@@ -590,8 +592,8 @@ int dump_call_grouped(XGPUContext *ctx, Internal *in, int b, int groups) {
       XGPU_CHECK(cudaEventRecord(in->group_out[k], in->s_comp));
       XGPU_CHECK(cudaStreamWaitEvent(in->s_dump, in->group_out[k], 0));
     }
-    XGPU_CHECK(launch_format(in->d_state, in->int_state ? 0 : 1, s, in->cfg.matrix_order,
-                             in->cfg.output_type, direct ? direct : in->d_out, s_fmt, f0, fc));
+    XGPU_CHECK(launch_format(in->d_state, in->int_state ? 0 : 1, s, dump_out(in, direct), s_fmt, f0,
+                             fc, direct != nullptr));
     if (!direct) XGPU_CHECK(cudaEventRecord(in->group_out[k], in->s_comp));
   }
   in->state_zero = false;
@@ -626,7 +628,6 @@ int finish_call(XGPUContext *ctx, Internal *in, int syncOp) {
       XGPU_CHECK(cudaStreamSynchronize(in->s_copy));
       return XGPU_OK;
     case SYNCOP_SYNC_COMPUTE:
-      XGPU_CHECK(cudaStreamSynchronize(in->s_comp));
       return check_device_error(in);
     default:
       return XGPU_OK;
@@ -784,8 +785,8 @@ int xgpuInitEx(XGPUContext *context, int device_flags, const XGPUConfig *cfg_in)
       cudaMalloc(&in->d_in[1], in_bytes) != cudaSuccess ||
       cudaMalloc(&in->d_state, state_bytes) != cudaSuccess ||
       cudaMalloc(&in->d_out, (size_t)s.mat_length * sizeof(Complex)) != cudaSuccess ||
-      cudaMalloc(&in->d_err, sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&in->h_err, sizeof(int)) != cudaSuccess ||
+      cudaHostGetDevicePointer((void **)&in->d_err, in->h_err, 0) != cudaSuccess ||
       (cfg.input_format != XGPU_INPUT_INT8 &&
        (cudaMalloc(&in->d_conv[0], (size_t)(2 * s.vec_length + 255) / 256 * 256) != cudaSuccess ||
         cudaMalloc(&in->d_conv[1], (size_t)(2 * s.vec_length + 255) / 256 * 256) != cudaSuccess ||
@@ -822,8 +823,8 @@ int xgpuInitEx(XGPUContext *context, int device_flags, const XGPUConfig *cfg_in)
       return fail(XGPU_CUDA_ERROR);
     }
   }
-  if (cudaMemsetAsync(in->d_err, 0, sizeof(int), in->s_comp) != cudaSuccess ||
-      cudaMemsetAsync(in->d_state, 0, state_bytes, in->s_comp) != cudaSuccess ||
+  *in->h_err = 0;
+  if (cudaMemsetAsync(in->d_state, 0, state_bytes, in->s_comp) != cudaSuccess ||
       cudaStreamSynchronize(in->s_comp) != cudaSuccess)
     return fail(XGPU_CUDA_ERROR);
   in->state_zero = true;
@@ -1037,12 +1038,10 @@ int xgpuDumpDeviceIntegrationBufferInt64(XGPUContext *context, long long *host_o
     if (r != XGPU_OK) return r;
   }
   if (in->state_zero) {
-    XGPU_CHECK(cudaStreamSynchronize(in->s_comp));
     memset(host_out, 0, bytes);
     return check_device_error(in);
   }
   XGPU_CHECK(cudaMemcpyAsync(host_out, in->d_state, bytes, cudaMemcpyDeviceToHost, in->s_comp));
-  XGPU_CHECK(cudaStreamSynchronize(in->s_comp));
   return check_device_error(in);
 }
 

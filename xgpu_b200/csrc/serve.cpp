@@ -437,7 +437,8 @@ extern "C" int xgpuServeRun(const XGPUServeJob *jobs, int njobs, const XGPUServe
           if (last) a.finished = true;
           if (last || (j.dump_every && (a.next_block % j.dump_every) == 0)) {
             // format on the step stream, copy on the dump stream
-            SCHECK(launch_format(a.state, 0, a.s, TRIANGULAR_ORDER, XGPU_INT32, a.dump, s_step));
+            const DumpOut out{(uint32_t *)a.dump, a.s.mat_length, TRIANGULAR_ORDER, XGPU_INT32};
+            SCHECK(launch_format(a.state, 0, a.s, out, s_step));
             cudaEvent_t fe = get_event();
             SCHECK(cudaEventRecord(fe, s_step));
             SCHECK(cudaStreamWaitEvent(s_dump, fe, 0));

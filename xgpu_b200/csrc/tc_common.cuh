@@ -166,6 +166,12 @@ __device__ __forceinline__ void tmem_ld128(uint32_t taddr, uint32_t (&v)[4][32])
   tmem_regs_after_wait(v[3]);
 }
 
+// Report a device error (one of DeviceError): err may be device memory or
+// page-locked host memory that the device maps.
+__device__ __forceinline__ void report_error(int *err, int code) {
+  *(volatile int *)err = code;
+}
+
 // Programmatic dependent launch.  pdl_trigger lets the next kernel of the
 // stream start its prologue now; pdl_wait blocks until the previous kernel of
 // the stream (when this one was launched programmatically) has completed and
