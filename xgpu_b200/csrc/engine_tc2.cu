@@ -823,16 +823,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPacked ? kThreadsPa
 // int64 buffer holds nothing yet) -- 2 KB contiguous, four 512-byte loads and
 // stores per warp, all loads first.  Rows i < n, columns j <= i only (the
 // block's other entries hold nothing).  Each int64 value has one writer.  The
-// words are left as they are: the next launch that uses them stores its own
-// (or they are cleared first).  Launched programmatically behind the engine
-// launch that filled the words: it waits for that launch (and so for the
-// chain before it) before touching memory, and lets the next launch start its
-// prologue at once.
+// words are left zero (zero_words), or as they are: the next launch that uses
+// them then stores its own (or they are cleared first).  Launched
+// programmatically behind the engine launch that filled the words: it waits for
+// that launch (and so for the chain before it) before touching memory, and lets
+// the next launch start its prologue at once.
 constexpr int kFoldColWords = 36;
-__global__ void __launch_bounds__(256) fold_words_kernel(const uint64_t *__restrict__ words,
+__global__ void __launch_bounds__(256) fold_words_kernel(uint64_t *__restrict__ words,
                                                          int64_t *__restrict__ state, int n,
                                                          long long nbaseline, int nblk,
-                                                         int store_state) {
+                                                         int store_state, int zero_words) {
   __shared__ __align__(16) unsigned long long sw[32 * kFoldColWords];
   pdl_wait();
   pdl_trigger();
@@ -841,10 +841,11 @@ __global__ void __launch_bounds__(256) fold_words_kernel(const uint64_t *__restr
   while (rb * (rb + 1) / 2 > k) --rb;
   while ((rb + 1) * (rb + 2) / 2 <= k) ++rb;
   const int cb = k - rb * (rb + 1) / 2;
-  const ulonglong2 *src =
-      reinterpret_cast<const ulonglong2 *>(words + ((long long)f * nblk + k) * 4096 + q * 1024);
+  ulonglong2 *src =
+      reinterpret_cast<ulonglong2 *>(words + ((long long)f * nblk + k) * 4096 + q * 1024);
   const int t = threadIdx.x;
   const ulonglong2 a0 = src[t], a1 = src[t + 256];   // words 2t, 2t+1 and 512 + 2t, 513 + 2t
+  if (zero_words) src[t] = src[t + 256] = make_ulonglong2(0, 0);
   const int ilq = t >> 5, lane = t & 31;
   const long long i = (long long)rb * kStations + q * 8 + ilq;
   const bool row_live = i < n;
@@ -898,6 +899,38 @@ bool tc2_single_item(int tcount, const TcTuning &tune) {
   return (total_steps + per - 1) / per == 1;
 }
 
+// Calls of a chain overlap, so a call need not fill the GPU by itself, and on
+// part of the SMs each CTA pair has more tiles, over which its prologue, first
+// loads and last drain (about 7 us together) spread.  But a call takes the
+// longer for it, and the last ones of a chain pay that.  So a pair gets about
+// 128 stages of 128 samples (some 55 us), the last call's, behind which nothing
+// overlaps, 32, and the call that has `before` others before it runs on at least
+// 1 / (before + 1) of the pairs, down to a quarter.  Chains of 4, 8 and 32 calls
+// and the wait for them, against single CTAs on every SM (pairs from 384
+// stations on): N=256, F=10, T=1024 73 to 68, 122 to 94 and 408 to 246 us;
+// N=128, F=64, T=2048 146 to 132, 270 to 240, 994 to 775; N=64, F=64, T=4096 106
+// to 103, 185 to 156, 621 to 508; N=512, F=4, T=2048 109 to 105, 193 to 167, 680
+// to 555.  (96 or 192 stages a pair: within 3% over 14 shapes; without the
+// growing share a chain of four loses up to 15%.)  Calls of fewer than 200
+// stages keep the context's default: the host queues them no faster than that
+// runs, and the fold before a dump is then lost (N=32, F=2, T=544: 110 us for 25
+// calls and a dump, 115 with pairs).
+TcTuning tc2_chain_tuning(const Sizes &s, const TcTuning &own, int before, bool last) {
+  const long long ntl = (4LL * s.n + 2 * tc2::kHalf - 1) / (2 * tc2::kHalf);
+  const long long steps = ntl * (ntl + 1) / 2 * s.f * ((s.t + tc2::kKt - 1) / tc2::kKt);
+  if (steps < 200) return own;
+  TcTuning t;
+  t.wide = 1;
+  t.stall = own.stall;
+  const int pairs = current_device_sms() / 2, part = before < 3 ? before + 1 : 4;
+  const int each = last ? 32 : 128;
+  long long k = (steps + each - 1) / each;
+  if (k < pairs / part) k = pairs / part;
+  if (k > pairs) k = pairs;
+  t.grid = (int)(2 * k);
+  return t;
+}
+
 long long words_blocks(const Sizes &s) {
   const long long nb = (s.n + tc2::kStations - 1) / tc2::kStations;
   return nb * (nb + 1) / 2;
@@ -905,8 +938,8 @@ long long words_blocks(const Sizes &s) {
 
 long long words_elems(const Sizes &s) { return (long long)s.f * words_blocks(s) * 4096; }
 
-cudaError_t launch_fold_words(const uint64_t *words, int64_t *state, const Sizes &s,
-                              cudaStream_t st, int overlap, int store_state) {
+cudaError_t launch_fold_words(uint64_t *words, int64_t *state, const Sizes &s,
+                              cudaStream_t st, int overlap, int store_state, int zero_words) {
   if (s.f > 65535) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(4 * words_blocks(s)), (unsigned)s.f);
@@ -918,7 +951,7 @@ cudaError_t launch_fold_words(const uint64_t *words, int64_t *state, const Sizes
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, tc2::fold_words_kernel, words, state, s.n, s.nbaseline,
-                            (int)words_blocks(s), store_state);
+                            (int)words_blocks(s), store_state, zero_words);
 }
 
 cudaError_t tc2_set_smem_attribute() {

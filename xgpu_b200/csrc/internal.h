@@ -110,7 +110,7 @@ cudaError_t launch_tc2(const CUtensorMap &map, const Sizes &s, int t0, int tcoun
                        int overwrite, int *err, cudaStream_t st, const TcTuning &tune,
                        int overlap, int f0 = 0, int fcount = -1,
                        const void *packed_in = nullptr, uint64_t *words = nullptr,
-                       int words_store = 0);
+                            int words_store = 0);
 // Word buffer: 64-bit words (im * 2^32 + re of one visibility's sums) in
 // 32 x 32-station blocks; its size for sizes s, and the fold that adds the
 // words into the int64 buffer (triangular order).  Exact while every sum in
@@ -121,6 +121,10 @@ long long words_blocks(const Sizes &s);   // 32-station blocks per channel
 // per tile (no time splits: it may store its words).
 bool tc2_uses_words(int tcount, const TcTuning &tune);
 bool tc2_single_item(int tcount, const TcTuning &tune);
+// The setting for a call of a chain that overlap one another, with `before` calls
+// ahead of it (CTA pairs on part of the SMs, or the context's own); last: the
+// caller waits for it.
+TcTuning tc2_chain_tuning(const Sizes &s, const TcTuning &own, int before, bool last);
 long long words_elems(const Sizes &s);
 // A dump's destination: matLength Complex as 32-bit words.
 struct DumpOut {
@@ -131,8 +135,10 @@ struct DumpOut {
 // overlap: the launch before it on `st` is an engine launch of the same
 // context (it may then start while that launch finishes).  store_state: the
 // int64 buffer holds nothing yet; the fold stores into it instead of adding.
-cudaError_t launch_fold_words(const uint64_t *words, int64_t *state, const Sizes &s,
-                              cudaStream_t st, int overlap = 0, int store_state = 0);
+// zero_words: leave the words zero.
+cudaError_t launch_fold_words(uint64_t *words, int64_t *state, const Sizes &s,
+                              cudaStream_t st, int overlap = 0, int store_state = 0,
+                              int zero_words = 0);
 constexpr int kWordsMaxSamples = 65535;
 // A batch of jobs from a device-resident table (item_begin ascending); with a
 // queue (device int) the CTAs take items dynamically, otherwise by stride.

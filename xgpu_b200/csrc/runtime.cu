@@ -115,6 +115,11 @@ struct Internal {
   int cur = 0;
   bool state_zero = true;
   TcTuning tune;   // tensor-core kernel, time splits and grid
+  bool tuned = false;   // chosen by xgpuTune: every call uses it
+  TcTuning use;         // the setting of the call in hand (call_tuning)
+  // Calls over device input queued on the context's own stream since the host
+  // last waited for it, or cleared or dumped the integration.
+  int chain = 0;
   // The last operation queued on s_comp is an engine launch that only added
   // into the integration buffer (no store), on the context's own stream: the
   // next accumulating launch over other input may overlap it.
@@ -276,7 +281,21 @@ const CUtensorMap *tensor_map(Internal *in, const void *ptr, const Sizes &g, boo
 // pre-pass.
 bool packed_in_kernel(const Internal *in) {
   return in->cfg.input_format == XGPU_INPUT_PACKED4 && in->int_state &&
-         in->cfg.engine == XGPU_ENGINE_TENSOR && in->tune.wide;
+         in->cfg.engine == XGPU_ENGINE_TENSOR && in->use.wide;
+}
+
+// The tensor engine's setting for a call over device input.  What xgpuTune chose
+// holds for every call.  Otherwise a call that follows others the host has not
+// waited for is one of a chain, which CTA pairs on part of the SMs run faster
+// where the calls may overlap (tc2_chain_tuning); the first one, which may stay
+// alone, uses the context's default.
+TcTuning call_tuning(const Internal *in, bool waited) {
+  const bool overlaps = in->s_comp == in->s_own && (in->cfg.input_format == XGPU_INPUT_INT8 ||
+                                                    in->cfg.input_format == XGPU_INPUT_PACKED4);
+  if (in->tuned || !in->int_state || in->cfg.engine != XGPU_ENGINE_TENSOR || in->chain == 0 ||
+      !overlaps)
+    return in->tune;
+  return tc2_chain_tuning(in->szc, in->tune, in->chain, waited);
 }
 
 // Queue the engine over channels [f0, f0 + fcount) of int8 input x (packed
@@ -284,7 +303,14 @@ bool packed_in_kernel(const Internal *in) {
 // first segment stores when the buffer is known to be zero.  x has geometry s
 // (in->szc for the context's compact buffers, in->sz for a full-band device
 // input read in place, x then pointing at the context's first channel).
-// Add the words into the int64 buffer (and zero them), on s_comp after
+// Word buffers up to this size are left zero by a fold.  The first launch after
+// it then adds, and the second overlaps it, which a launch that stores its words
+// does not allow: N=256, F=10 (11.8 MB), 32 calls and a dump on 36 CTAs, 475 to
+// 457 us.  Larger ones cost more to zero, and to add to, than their longer calls
+// gain (N=496, F=11, 49 MB: two calls and a dump 920 to 946 us).
+constexpr long long kZeroWords = (24 << 20) / 8;
+
+// Add the words into the int64 buffer, on s_comp after
 // everything queued there: before the buffer is read, and before the words
 // would hold more than kWordsMaxSamples samples.  after_adding: the last
 // launch on s_comp is an adding engine launch of this context, which the fold
@@ -292,13 +318,14 @@ bool packed_in_kernel(const Internal *in) {
 // engine launch does not overlap the fold; it only starts its prologue early.
 int fold_words(Internal *in, bool after_adding = false) {
   if (!in->words_dirty) return XGPU_OK;
+  const bool zero = words_elems(in->szc) <= kZeroWords;
   // an integration held only in the words is stored into d_state
   XGPU_CHECK(launch_fold_words(in->d_words, (int64_t *)in->d_state, in->szc, in->s_comp,
                                after_adding && in->s_comp == in->s_own ? 1 : 0,
-                               in->state_zero ? 1 : 0));
+                               in->state_zero ? 1 : 0, zero ? 1 : 0));
   in->state_zero = false;
   in->words_dirty = false;
-  in->words_stale = true;
+  in->words_stale = !zero;
   in->words_samples = 0;
   in->adding_tail = false;
   return XGPU_OK;
@@ -335,11 +362,11 @@ int launch_engine(Internal *in, const int8_t *x, const Sizes &s, int f0, int fco
     bool state_written = false;
     for (int t0 = 0; t0 < s.t; t0 += kSegment) {
       const int tc = s.t - t0 < kSegment ? s.t - t0 : kSegment;
-      const bool words = allow_words && in->d_words && in->tune.wide && tc2_uses_words(tc, in->tune);
+      const bool words = allow_words && in->d_words && in->use.wide && tc2_uses_words(tc, in->use);
       if (!words) {
         const int store = in->state_zero && !state_written ? 1 : 0;
         XGPU_CHECK(launch_tc_tuned(*map, s, t0, tc, (int64_t *)in->d_state, store, in->d_err,
-                                   in->s_comp, in->tune, *tail && !store ? 1 : 0, f0, fcount,
+                                   in->s_comp, in->use, *tail && !store ? 1 : 0, f0, fcount,
                                    packed ? (const void *)x : nullptr));
         state_written = true;
         *tail = !store;   // the next segment follows an adding launch
@@ -350,19 +377,20 @@ int launch_engine(Internal *in, const int8_t *x, const Sizes &s, int f0, int fco
         if (r != XGPU_OK) return r;
         *tail = false;
       }
-      // Words that hold nothing are overwritten by a launch with one item per
-      // tile; a launch with time splits adds, into words cleared first.
+      // Words that hold nothing but are not zero are overwritten by a launch
+      // with one item per tile; a launch with time splits adds, into words
+      // cleared first.
       int wstore = 0;
-      if (!in->words_dirty) {
-        if (tc2_single_item(tc, in->tune)) {
+      if (in->words_stale) {
+        if (tc2_single_item(tc, in->use)) {
           wstore = 1;
-        } else if (in->words_stale) {
+        } else {
           XGPU_CHECK(cudaMemsetAsync(in->d_words, 0, (size_t)words_elems(in->szc) * 8, in->s_comp));
           *tail = false;
         }
       }
       XGPU_CHECK(launch_tc_tuned(*map, s, t0, tc, (int64_t *)in->d_state, 0, in->d_err, in->s_comp,
-                                 in->tune, *tail && !wstore ? 1 : 0, f0, fcount,
+                                 in->use, *tail && !wstore ? 1 : 0, f0, fcount,
                                  packed ? (const void *)x : nullptr, in->d_words, wstore));
       in->words_samples += tc;
       in->words_dirty = true;
@@ -380,8 +408,9 @@ int launch_engine(Internal *in, const int8_t *x, const Sizes &s, int f0, int fco
 // compact: d_input holds only this context's channels (the copy the host path
 // makes); otherwise it is the caller's full-band input, read in place (int8,
 // or packed input the CTA-pair kernel expands) or gathered into d_slice
-// before its conversion (the other formats).
-int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool compact) {
+// before its conversion (the other formats).  allow_words: as launch_engine's.
+int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool compact,
+               bool allow_words = true) {
   const Sizes &s = in->sz;
   const bool ranged = !compact && s.fin != s.f;
   const int8_t *x = (const int8_t *)d_input;
@@ -431,7 +460,7 @@ int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool 
     }
   }
   bool wrote_state = true;
-  const int r = launch_engine(in, x, *geom, 0, s.f, &tail, packed, true, &wrote_state);
+  const int r = launch_engine(in, x, *geom, 0, s.f, &tail, packed, allow_words, &wrote_state);
   if (r != XGPU_OK) return r;
   if (in->int_state) in->adding_tail = tail && conv < 0;   // tensor or dp4a engine
   if (wrote_state) in->state_zero = false;   // otherwise the call went to the words
@@ -446,6 +475,7 @@ int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool 
 // launch's), then read and clear the device error word.
 int check_device_error(Internal *in, cudaStream_t st = nullptr) {
   in->adding_tail = false;
+  in->chain = 0;
   XGPU_CHECK(cudaStreamSynchronize(st ? st : in->s_comp));
   const int err = *(volatile int *)in->h_err;
   if (err != 0) {
@@ -863,6 +893,7 @@ int xgpuClearDeviceIntegrationBuffer(XGPUContext *context) {
     in->words_samples = 0;
   }
   in->adding_tail = false;
+  in->chain = 0;
   in->state_zero = true;
   return XGPU_OK;
 }
@@ -979,6 +1010,8 @@ int xgpuCudaXengine(XGPUContext *context, int syncOp) {
     return XGPU_INVALID_ARGUMENT;
   XGPU_CHECK(cudaSetDevice(in->device));
 
+  in->use = in->tune;
+  in->chain = 0;
   const int b = in->cur;
   in->cur ^= 1;
   if (syncOp == SYNCOP_DUMP) {
@@ -1013,8 +1046,14 @@ int xgpuCudaXengineDevice(XGPUContext *context, const void *device_input, int sy
   if (!device_input || ((uintptr_t)device_input & 15) != 0) return XGPU_INVALID_ARGUMENT;
   if (syncOp < SYNCOP_NONE || syncOp > SYNCOP_SYNC_COMPUTE) return XGPU_INVALID_ARGUMENT;
   XGPU_CHECK(cudaSetDevice(in->device));
-  int r = run_engine(in, device_input, nullptr, false);
+  in->use = call_tuning(in, syncOp != SYNCOP_NONE);
+  // A call that the host waits for, with none before it, goes to the int64 buffer
+  // itself: the words' fold would follow at once (N=736, F=18, T=912, one call
+  // and its dump: 3.18 ms with words, 3.08 without).
+  const bool words = syncOp == SYNCOP_NONE || in->chain > 0 || in->words_dirty;
+  int r = run_engine(in, device_input, nullptr, false, words);
   if (r != XGPU_OK) return r;
+  ++in->chain;
   return finish_call(context, in, syncOp);
 }
 
@@ -1059,6 +1098,7 @@ int xgpuSetComputeStream(XGPUContext *context, void *stream) {
   cudaStream_t next = stream ? (cudaStream_t)stream : in->s_own;
   if (next == in->s_comp) return XGPU_OK;
   in->adding_tail = false;
+  in->chain = 0;
   // Order the new stream after everything queued on the old one.
   cudaEvent_t ev;
   XGPU_CHECK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
@@ -1080,6 +1120,7 @@ int xgpuTune(XGPUContext *context, int ksplit, int grid, int pair) {
   if (ksplit < 0 || grid < 0 || pair < 0 || pair > 2) return XGPU_INVALID_ARGUMENT;
   in->adding_tail = false;
   if (ksplit > 0) {
+    in->tuned = true;
     in->tune.ksplit = ksplit;
     in->tune.grid = grid;
     in->tune.wide = pair == 1 ? 1 : 0;
@@ -1238,6 +1279,7 @@ int xgpuTune(XGPUContext *context, int ksplit, int grid, int pair) {
   if (rot) cudaFree(rot);
   if (rc != XGPU_OK) return rc;
   in->tune = best_t;
+  in->tuned = true;
   return check_device_error(in);
 }
 
