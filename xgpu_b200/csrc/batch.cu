@@ -6,8 +6,8 @@
 // Gram matrix), writes the job table to device memory once, and runs all
 // items in one launch of the persistent tensor-core kernel, whose CTAs take
 // items from a global atomic queue so long and short jobs balance across the
-// SMs.  Plans are captured once into a CUDA graph (queue reset, buffer clears,
-// kernel) and replayed.  An autotuner picks the time-split granularity and the
+// SMs.  Plans are captured once into a CUDA graph (buffer clears, kernel) and
+// replayed.  An autotuner picks the time-split granularity and the
 // grid size by timing the batch on scratch integration buffers.
 //
 // xGPU has no counterpart: it runs one compile-time shape per library build
@@ -264,13 +264,14 @@ int xgpuBatchCreate(XGPUBatch *out, const XGPUBatchJob *jobs, int njobs, int dev
     return fail(XGPU_CUDA_ERROR);
   }
   if (cudaMalloc(&b->d_jobs, njobs * sizeof(Job)) != cudaSuccess ||
-      cudaMalloc(&b->d_queue, sizeof(int)) != cudaSuccess ||
+      cudaMalloc(&b->d_queue, 2 * sizeof(int)) != cudaSuccess ||
       cudaMalloc(&b->d_err, sizeof(int)) != cudaSuccess ||
       cudaMallocHost(&b->h_err, sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
     return fail(XGPU_OUT_OF_MEMORY);
   }
-  if (cudaMemsetAsync(b->d_err, 0, sizeof(int), b->stream) != cudaSuccess)
+  if (cudaMemsetAsync(b->d_err, 0, sizeof(int), b->stream) != cudaSuccess ||
+      cudaMemsetAsync(b->d_queue, 0, 2 * sizeof(int), b->stream) != cudaSuccess)
     return fail(XGPU_CUDA_ERROR);
   b->grid = num_sms(device);
   b->max_steps = 0;
@@ -286,7 +287,7 @@ int xgpuBatchCreate(XGPUBatch *out, const XGPUBatchJob *jobs, int njobs, int dev
   if (r != XGPU_OK) return fail(r);
   if ((r = upload(b, table, b->d_jobs)) != XGPU_OK) return fail(r);
   if (flags & XGPU_BATCH_GRAPH) {
-    // Capture clears, queue reset and the kernel once; xgpuBatchRun replays.
+    // Capture clears and the kernel once; xgpuBatchRun replays.
     cudaStream_t cs;
     if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess)
       return fail(XGPU_CUDA_ERROR);

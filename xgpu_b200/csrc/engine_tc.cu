@@ -72,7 +72,7 @@ struct Params {
   const Job *jobs;     // batched: job table in global memory, ordered by item_begin
   int njobs;
   int total;           // work items over all jobs
-  int *queue;          // dynamic work counter (zeroed before launch); nullptr: static stride
+  int *queue;          // work queue (queue_claim); nullptr: static stride
   int *err;
   int stall;           // test switch: issue no loads (the waits on them expire)
   int streamk;         // single job: each CTA takes an equal share of all (tile, stage) steps
@@ -216,6 +216,7 @@ __global__ void __launch_bounds__(kThreads, 1) xengine_tc_kernel(const __grid_co
       if (!p.jobs) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&p.single.map) : "memory");
       uint32_t g = 0, g_loaded = 0;
       bool ok = true;
+      int next = (int)blockIdx.x;   // the next item
       // Stream-K: CTA b covers steps [b*W/G, (b+1)*W/G) of the W = items x
       // stages of the job, cutting tiles where the ranges meet; the pieces of
       // a cut tile add up exactly in the integration buffer (reduce-add).
@@ -245,7 +246,8 @@ __global__ void __launch_bounds__(kThreads, 1) xengine_tc_kernel(const __grid_co
             t.u = p.total;
           }
         } else {
-          const int u = p.queue ? atomicAdd(p.queue, 1) : (int)blockIdx.x + i * (int)gridDim.x;
+          const int u = next;
+          next = u + (int)gridDim.x;
           if (u < p.total) {
             t = decode_item(p, u);
           } else {
@@ -258,6 +260,10 @@ __global__ void __launch_bounds__(kThreads, 1) xengine_tc_kernel(const __grid_co
         if (u >= p.total) break;
         const bool diag = (t.tr == t.tc);
         const CUtensorMap *map = t.map;
+        // The stage at whose load the next item is claimed: a few before the
+        // item's last, so that the claim's way to memory and back passes under
+        // the loads.
+        const int claim = !p.queue ? -1 : t.nsteps > 4 ? t.nsteps - 4 : 0;
         for (int ks = 0; ks < t.nsteps; ++ks, ++g) {
           const uint32_t s = g % kStages;
           if (g >= (uint32_t)kStages &&
@@ -266,6 +272,7 @@ __global__ void __launch_bounds__(kThreads, 1) xengine_tc_kernel(const __grid_co
             ok = false;
             break;
           }
+          if (ks == claim) next = queue_claim(p.queue, (int)gridDim.x);
           if (p.stall) continue;
           const uint32_t dst = stage0 + s * kStageBytes;
           mbar_expect_tx(full0 + 8 * s, diag ? kBoxBytes : 2 * kBoxBytes);
@@ -275,6 +282,7 @@ __global__ void __launch_bounds__(kThreads, 1) xengine_tc_kernel(const __grid_co
           g_loaded = g + 1;
         }
       }
+      if (p.queue) queue_done(p.queue, (int)gridDim.x);
       // Loads still in flight land before the CTA leaves (a no-op normally).
       for (uint32_t q = (g_loaded > (uint32_t)kStages ? g_loaded - kStages : 0); q < g_loaded; ++q)
         mbar_wait(full0 + 8 * (q % kStages), (q / kStages) & 1, nullptr);
@@ -618,10 +626,10 @@ cudaError_t launch_tc_batch(const Job *dev_jobs, int njobs, int total_items, int
   if (!sms) return cudaErrorInvalidDevice;
   cudaError_t e = tc_configure_device();
   if (e != cudaSuccess) return e;
-  if (queue) {
-    e = cudaMemsetAsync(queue, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
-  }
+  if (grid <= 0) grid = sms;
+  if (grid > total_items) grid = total_items;
+  if (grid < 1) return cudaSuccess;
+  if (grid == total_items) queue = nullptr;   // one item each: nothing to balance
   tc::Params p;
   memset(&p.single, 0, sizeof(p.single));
   p.jobs = dev_jobs;
@@ -632,9 +640,6 @@ cudaError_t launch_tc_batch(const Job *dev_jobs, int njobs, int total_items, int
   p.stall = 0;
   p.streamk = 0;
   p.overlap = 0;
-  if (grid <= 0) grid = sms;
-  if (grid > total_items) grid = total_items;
-  if (grid < 1) return cudaSuccess;
   tc::xengine_tc_kernel<<<grid, tc::kThreads, tc::kSmemBytes, st>>>(p);
   return cudaGetLastError();
 }

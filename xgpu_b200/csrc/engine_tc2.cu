@@ -101,7 +101,7 @@ struct Params {
   const Job *jobs;     // batched: job table in global memory, ordered by item_begin
   int njobs;
   int total;           // work items over all jobs
-  int *queue;          // dynamic work counter (zeroed before launch); nullptr: static stride
+  int *queue;          // work queue (queue_claim); nullptr: static stride
   int *err;
   int stall;           // test switch: issue no loads (the waits on them expire)
   int overlap;         // may run alongside the previous (accumulating) launch of the stream
@@ -399,16 +399,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPacked ? kThreadsPa
       if (!p.jobs && leader) asm volatile("prefetch.tensormap [%0];" ::"l"((uint64_t)&p.job.map) : "memory");
       uint32_t g = 0;
       bool ok = true;
+      int next = cid;   // the leader's next item
       for (int i = 0; ok; ++i) {
         const int slot = i % kSched;
         Item t;
+        int claim = -1;   // the stage at whose load the next item is claimed from the queue
         if (leader) {
           if (i >= kSched && !mbar_wait(sempty0 + 8 * slot, ((i / kSched) - 1) & 1, abort_flag)) {
             fail(kErrTimeoutProducer);
             break;
           }
-          const int u = p.queue ? atomicAdd(p.queue, 1) : cid + i * ncl;
+          const int u = next;
           if (u < p.total) t = decode(p, u); else t.u = u;
+          next = u + ncl;
+          // a few stages before the item's last load, so that the claim's way to
+          // memory and back passes under the loads
+          if (p.queue && u < p.total) claim = t.nsteps > 4 ? t.nsteps - 4 : 0;
           ring[slot] = t;
           const uint32_t remote = peer_addr(smem_u32(&ring[slot]), 1);
 #pragma unroll
@@ -455,6 +461,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPacked ? kThreadsPa
               ok = false;
               break;
             }
+            if (ks == claim) next = queue_claim(p.queue, ncl);
             if (p.stall) continue;
             const uint32_t dst = stage0 + s * kStageBytes;
             const int z = t.t0 + (t.step0 + ks) * kKt;
@@ -467,6 +474,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPacked ? kThreadsPa
           }
         }
       }
+      if (p.queue && leader) queue_done(p.queue, ncl);
       if (kPacked && ok && !p.stall) {
         // No stage follows: one slot says so to every converter warp.
         const uint32_t q = g % kPackedSlots;
@@ -1043,10 +1051,10 @@ cudaError_t launch_tc2_batch(const Job *dev_jobs, int njobs, int total_items, in
   if (!sms) return cudaErrorInvalidDevice;
   cudaError_t e = tc_configure_device();
   if (e != cudaSuccess) return e;
-  if (queue) {
-    e = cudaMemsetAsync(queue, 0, sizeof(int), st);
-    if (e != cudaSuccess) return e;
-  }
+  int clusters = (grid > 0 ? grid : sms) / 2;
+  if (clusters > total_items) clusters = total_items;
+  if (clusters < 1) return cudaSuccess;
+  if (clusters == total_items) queue = nullptr;   // one item each: nothing to balance
   tc2::Params p;
   memset(&p.job, 0, sizeof(p.job));
   p.jobs = dev_jobs;
@@ -1060,9 +1068,6 @@ cudaError_t launch_tc2_batch(const Job *dev_jobs, int njobs, int total_items, in
   p.words_nblk = 0;
   p.words_store = 0;
   p.split_epi = max_item_steps <= tc2::kSplitEpilogueSteps ? 1 : 0;
-  int clusters = (grid > 0 ? grid : sms) / 2;
-  if (clusters > total_items) clusters = total_items;
-  if (clusters < 1) return cudaSuccess;
   tc2::xengine_tc2_kernel<false><<<2 * clusters, tc2::kThreads, tc2::kSmemBytes, st>>>(p);
   return cudaGetLastError();
 }

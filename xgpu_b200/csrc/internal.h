@@ -141,7 +141,8 @@ cudaError_t launch_fold_words(uint64_t *words, int64_t *state, const Sizes &s,
                               int zero_words = 0);
 constexpr int kWordsMaxSamples = 65535;
 // A batch of jobs from a device-resident table (item_begin ascending); with a
-// queue (device int) the CTAs take items dynamically, otherwise by stride.
+// queue (two device ints, zero at first; every launch leaves them zero) the CTAs
+// take items dynamically, otherwise by stride.
 cudaError_t launch_tc_batch(const Job *dev_jobs, int njobs, int total_items, int *queue, int *err,
                             int grid, cudaStream_t st);
 // Fill a job for samples [t0, t0+tcount) of dev_in (sizes s).  store=1 asks for

@@ -251,7 +251,8 @@ extern "C" int xgpuServeRun(const XGPUServeJob *jobs, int njobs, const XGPUServe
   SCHECK(cudaStreamCreateWithFlags(&s_dump, cudaStreamNonBlocking));
   SCHECK(cudaMalloc(&d_tables, sizeof(Job) * max_table * kTables));
   SCHECK(cudaMallocHost(&h_tables, sizeof(Job) * max_table * kTables));
-  SCHECK(cudaMalloc(&d_queue, sizeof(int) * kTables));
+  SCHECK(cudaMalloc(&d_queue, 2 * sizeof(int) * kTables));
+  SCHECK(cudaMemsetAsync(d_queue, 0, 2 * sizeof(int) * kTables, s_step));
   SCHECK(cudaMalloc(&d_err, sizeof(int)));
   SCHECK(cudaMemsetAsync(d_err, 0, sizeof(int), s_step));
   {
@@ -422,7 +423,7 @@ extern "C" int xgpuServeRun(const XGPUServeJob *jobs, int njobs, const XGPUServe
           int max_steps = 0;
           for (int q = 0; q < nent; ++q)
             max_steps = tab[q].steps_per_split > max_steps ? tab[q].steps_per_split : max_steps;
-          SCHECK(launch_tc2_batch(dtab, nent, items, d_queue + table_slot, d_err, sms, s_step,
+          SCHECK(launch_tc2_batch(dtab, nent, items, d_queue + 2 * table_slot, d_err, sms, s_step,
                                   max_steps));
         }
         table_slot = (table_slot + 1) % kTables;
