@@ -378,17 +378,10 @@ __global__ void __launch_bounds__(kThreads, 1) xengine_tc_kernel(const __grid_co
       for (int q = 0; q < kTile / 32; ++q) {
 #pragma unroll
         for (int jj = 0; jj < 8; ++jj) {
-          // Columns 4jj..4jj+3: (p2=0 re, p2=0 im, p2=1 re, p2=1 im) of station
-          // j.  The real-row lane produces p2 = 0, the imaginary-row lane p2 = 1;
-          // each needs two values from its partner lane.
-          const int v0 = (int)v[q][4 * jj], v1 = (int)v[q][4 * jj + 1];
-          const int v2 = (int)v[q][4 * jj + 2], v3 = (int)v[q][4 * jj + 3];
-          const int ra = __shfl_xor_sync(0xffffffffu, c ? v0 : v2, 1);
-          const int rb = __shfl_xor_sync(0xffffffffu, c ? v1 : v3, 1);
-          const long long re = c ? (long long)ra + v3 : (long long)v0 + rb;
-          const long long im = c ? (long long)v2 - rb : (long long)ra - v1;
+          const int2 x = combine((int)v[q][4 * jj], (int)v[q][4 * jj + 1], (int)v[q][4 * jj + 2],
+                                 (int)v[q][4 * jj + 3], c);
           const int jl = q * 8 + jj;
-          if (jl < jmax) *(longlong2 *)(srow + jl * 64) = make_longlong2(re, im);
+          if (jl < jmax) *(int4 *)(srow + jl * 64) = make_int4(x.x, x.x >> 31, x.y, x.y >> 31);
         }
       }
       // Staging rows complete: hand them to the bulk-copy engine.

@@ -185,6 +185,22 @@ __device__ __forceinline__ void pdl_wait() {
 }
 
 
+// One visibility from the accumulator: a lane holds row (station i, p1, re or im:
+// c) of four columns v = (station j: p2 = 0 re, im, p2 = 1 re, im).  The real-row
+// lane makes product p2 = 0, the imaginary-row lane (its neighbour) p2 = 1; each
+// needs two values of the other:
+//   re = G(re, re) + G(im, im), im = G(im, re) - G(re, im).
+// In 32 bits: the accumulators hold at most kSegment samples, so that re and im
+// stay within 2^30; a third of the instructions of the 64-bit form.  A drain of
+// 128 columns, which four warps with nothing to hide behind spend on the
+// dependent instructions of this, took 1.65 us with that and takes 1.15.
+__device__ __forceinline__ int2 combine(int v0, int v1, int v2, int v3, bool c) {
+  const int r = __shfl_xor_sync(0xffffffffu, c ? v1 : v2, 1);
+  const int m = __shfl_xor_sync(0xffffffffu, c ? v0 : v3, 1);
+  const int d = m - (c ? v2 : v1);
+  return make_int2((c ? v3 : v0) + r, c ? -d : d);
+}
+
 // The work queue of a batch, two ints that are zero between launches: items
 // claimed beyond each CTA's (or CTA pair's) first, which is its own index, and
 // CTAs through with claiming.  The last of `takers` to be through zeroes both
