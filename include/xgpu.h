@@ -379,7 +379,8 @@ typedef struct XGPUBatchJobStruct {
 typedef struct XGPUBatchImpl *XGPUBatch;
 
 #define XGPU_BATCH_AUTOTUNE 1  /* time split granularity and grid chosen by timing */
-#define XGPU_BATCH_GRAPH    2  /* capture the run once as a CUDA graph and replay it */
+#define XGPU_BATCH_GRAPH    2  /* capture the run once as a CUDA graph and replay it (a run that
+                                  is one kernel launch is launched directly, which is faster) */
 #define XGPU_BATCH_PAIR     4  /* CTA-pair kernel, 256x256 tiles (without AUTOTUNE) */
 
 /* Plan a batch on `device`, run on `stream` (a cudaStream_t, NULL = legacy

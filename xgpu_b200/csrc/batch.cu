@@ -6,9 +6,10 @@
 // Gram matrix), writes the job table to device memory once, and runs all
 // items in one launch of the persistent tensor-core kernel, whose CTAs take
 // items from a global atomic queue so long and short jobs balance across the
-// SMs.  Plans are captured once into a CUDA graph (buffer clears, kernel) and
-// replayed.  An autotuner picks the time-split granularity and the
-// grid size by timing the batch on scratch integration buffers.
+// SMs.  Plans of more than the one launch (buffer clears before it) are captured
+// once into a CUDA graph and replayed.  An autotuner picks the time-split
+// granularity and the grid size by timing the batch on scratch integration
+// buffers.
 //
 // xGPU has no counterpart: it runs one compile-time shape per library build
 // (xgpu_info.h:6-25), so a mixed workload there is a loop of separate
@@ -286,8 +287,14 @@ int xgpuBatchCreate(XGPUBatch *out, const XGPUBatchJob *jobs, int njobs, int dev
   int r = build_table(b, states, b->max_steps, b->pair, table, b->total_items);
   if (r != XGPU_OK) return fail(r);
   if ((r = upload(b, table, b->d_jobs)) != XGPU_OK) return fail(r);
-  if (flags & XGPU_BATCH_GRAPH) {
-    // Capture clears and the kernel once; xgpuBatchRun replays.
+  // A run that is the kernel alone is launched as it is: consecutive launches
+  // overlap the next one's start with the last one's end, which replays of a graph
+  // do not (8 tiny subarrays: 10.3 us a run replayed, 8.7 launched; 3 up to N=400:
+  // 28.2 and 25.6).  A run with buffer clears before the kernel (time splits whose
+  // sums replace the buffer's) is captured once, and replayed.
+  bool clears = false;
+  for (size_t q = 0; q < table.size(); ++q) clears |= !b->jobs[q].accumulate && !table[q].store;
+  if ((flags & XGPU_BATCH_GRAPH) && clears) {
     cudaStream_t cs;
     if (cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking) != cudaSuccess)
       return fail(XGPU_CUDA_ERROR);

@@ -633,8 +633,18 @@ cudaError_t launch_tc_batch(const Job *dev_jobs, int njobs, int total_items, int
   p.stall = 0;
   p.streamk = 0;
   p.overlap = 0;
-  tc::xengine_tc_kernel<<<grid, tc::kThreads, tc::kSmemBytes, st>>>(p);
-  return cudaGetLastError();
+  // Programmatic: the prologue passes under the previous launch's end.
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3(tc::kThreads);
+  cfg.dynamicSmemBytes = tc::kSmemBytes;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, tc::xengine_tc_kernel, p);
 }
 
 }  // namespace xgpu

@@ -1066,8 +1066,18 @@ cudaError_t launch_tc2_batch(const Job *dev_jobs, int njobs, int total_items, in
   p.words_nblk = 0;
   p.words_store = 0;
   p.split_epi = max_item_steps <= tc2::kSplitEpilogueSteps ? 1 : 0;
-  tc2::xengine_tc2_kernel<false><<<2 * clusters, tc2::kThreads, tc2::kSmemBytes, st>>>(p);
-  return cudaGetLastError();
+  // Programmatic: the prologue passes under the previous launch's end.
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * clusters));
+  cfg.blockDim = dim3(tc2::kThreads);
+  cfg.dynamicSmemBytes = tc2::kSmemBytes;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, tc2::xengine_tc2_kernel<false>, p);
 }
 
 }  // namespace xgpu
