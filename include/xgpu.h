@@ -345,7 +345,8 @@ int xgpuCorrelateStatic(const void *device_input, void *device_output, const XGP
  * input from device memory rather than the L2 cache (temporary buffers of up
  * to about 256 MB plus one integration buffer, freed before it returns), and
  * the fastest setting is kept.  With CTA pairs, XGPU_INPUT_PACKED4 input
- * is expanded inside the kernel; the other kernels read an int8 copy that a
+ * is expanded inside the kernel, except for long calls, whose input a pre-pass
+ * converts beside the previous call; the other kernels read an int8 copy that a
  * pre-pass makes. */
 int xgpuTune(XGPUContext *context, int ksplit, int grid, int pair);
 

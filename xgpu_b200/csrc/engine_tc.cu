@@ -60,8 +60,8 @@ constexpr int kStageBytes = 2 * kBoxBytes;
 // Staging of one 32x32-station block of drained sums (staging_row).
 constexpr int kStateBytes = kStagingBytes;
 constexpr int kBarrierBytes = 512;    // barriers, work-item ring, TMEM slot
-constexpr int kSmemBytes = kStages * kStageBytes + kStateBytes + kBarrierBytes + 1024;
-static_assert(kSmemBytes <= 227 * 1024, "dynamic shared memory of one CTA");
+constexpr int kSmemBytes = kStages * kStageBytes + kStateBytes + kBarrierBytes;
+static_assert(kSmemBytes + 1024 <= kSmemBeside, "room for the next call's conversion");
 constexpr uint32_t kTmemCols = 2 * kTile;  // two accumulators
 constexpr int kThreads = 192;
 
@@ -149,8 +149,12 @@ __device__ __forceinline__ int64_t *row_ptr(const Item &t, int il) {
 }
 
 __global__ void __launch_bounds__(kThreads, 1) xengine_tc_kernel(const __grid_constant__ Params p) {
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  if (smem != smem_raw) {   // the swizzled boxes need the alignment, and there is no slack
+    report_error(p.err, kErrSharedBase);
+    return;
+  }
   uint8_t *sstate = smem + kStages * kStageBytes;
   uint64_t *bars = (uint64_t *)(sstate + kStateBytes);
   // full[kStages] empty[kStages] tfull[2] tempty[2] sfull[kSched] sempty[kSched] mma_done

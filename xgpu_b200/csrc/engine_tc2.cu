@@ -56,8 +56,8 @@ constexpr int kStageBytes = 2 * kBoxBytes;  // A rows + B half
 // Staging of one 32x32-station block of drained sums (staging_row).
 constexpr int kStateBytes = kStagingBytes;
 constexpr int kBarrierBytes = 512;    // barriers, work-item ring, TMEM slot
-constexpr int kSmemBytes = kStages * kStageBytes + kStateBytes + kBarrierBytes + 1024;
-static_assert(kSmemBytes <= 227 * 1024, "dynamic shared memory of one CTA");
+constexpr int kSmemBytes = kStages * kStageBytes + kStateBytes + kBarrierBytes;
+static_assert(kSmemBytes + 1024 <= kSmemBeside, "room for the next call's conversion");
 constexpr uint32_t kAccCols = 2 * kHalf;    // 256 columns per accumulator
 constexpr uint32_t kTmemCols = 2 * kAccCols;
 constexpr int kThreads = 192;
@@ -311,8 +311,12 @@ __device__ __forceinline__ void commit_pair(uint32_t cluster_bar) {
 template <bool kPacked>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPacked ? kThreadsPacked : kThreads, 1)
     xengine_tc2_kernel(const __grid_constant__ Params p) {
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  if (smem != smem_raw) {   // the swizzled boxes need the alignment, and there is no slack
+    report_error(p.err, kErrSharedBase);
+    return;
+  }
   // operand stages the MMA reads (packed input: the rest of the int8
   // kernel's stage memory holds the packed slots)
   constexpr int S = kPacked ? kStagesPacked : kStages;
@@ -905,6 +909,11 @@ bool tc2_single_item(int tcount, const TcTuning &tune) {
   return (total_steps + per - 1) / per == 1;
 }
 
+long long tc2_stages(const Sizes &s) {
+  const long long ntl = (4LL * s.n + 2 * tc2::kHalf - 1) / (2 * tc2::kHalf);
+  return ntl * (ntl + 1) / 2 * s.f * ((s.t + tc2::kKt - 1) / tc2::kKt);
+}
+
 // Calls of a chain overlap, so a call need not fill the GPU by itself, and on
 // part of the SMs each CTA pair has more tiles, over which its prologue, first
 // loads and last drain (about 7 us together) spread.  But a call takes the
@@ -917,14 +926,16 @@ bool tc2_single_item(int tcount, const TcTuning &tune) {
 // N=128, F=64, T=2048 146 to 132, 270 to 240, 994 to 775; N=64, F=64, T=4096 106
 // to 103, 185 to 156, 621 to 508; N=512, F=4, T=2048 109 to 105, 193 to 167, 680
 // to 555.  (96 or 192 stages a pair: within 3% over 14 shapes; without the
-// growing share a chain of four loses up to 15%.)  Calls of fewer than 200
+// growing share a chain of four loses up to 15%.)  A stage of packed input takes
+// half as long again.  Calls of fewer than 200
 // stages keep the context's default: the host queues them no faster than that
 // runs, and the fold before a dump is then lost (N=32, F=2, T=544: 110 us for 25
 // calls and a dump, 115 with pairs).
-TcTuning tc2_chain_tuning(const Sizes &s, const TcTuning &own, int before, bool last) {
-  const long long ntl = (4LL * s.n + 2 * tc2::kHalf - 1) / (2 * tc2::kHalf);
-  const long long steps = ntl * (ntl + 1) / 2 * s.f * ((s.t + tc2::kKt - 1) / tc2::kKt);
+TcTuning tc2_chain_tuning(const Sizes &s, const TcTuning &own, int before, bool last,
+                          bool packed) {
+  long long steps = tc2_stages(s);
   if (steps < 200) return own;
+  if (packed) steps += steps / 2;
   TcTuning t;
   t.wide = 1;
   t.stall = own.stall;

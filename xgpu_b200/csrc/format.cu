@@ -160,16 +160,41 @@ __global__ void __launch_bounds__(kHostThreads)
   }
 }
 
+// Conversions are programmatic launches between two engine launches.  Beside the
+// engine launch before it a conversion touches neither that one's input nor its
+// sums, so it starts at once and only ends after it (one block's wait keeps the
+// grid; the others leave their places to the rest); the engine launch behind it
+// waits for the conversion, and so for both.
+__device__ __forceinline__ void begin_conversion(int beside) {
+  if (!beside) tc::pdl_wait();
+  tc::pdl_trigger();
+}
+__device__ __forceinline__ void end_conversion(int beside) {
+  if (beside && blockIdx.x == 0) tc::pdl_wait();
+}
+
+// Item u of the compact input (rows of `row` items) in the caller's, whose rows
+// are `pitch` items apart: the band's, of which the context correlates a range.
+struct Rows {
+  long long row, pitch;
+  __device__ __forceinline__ long long at(long long u) const {
+    return row == pitch ? u : u / row * pitch + u % row;
+  }
+};
+
 // 16 packed samples per thread: one 16-byte load, two 16-byte stores.
-__global__ void unpack4_kernel(const uint4 *in, uint4 *out, long long nquads) {
+__global__ void unpack4_kernel(const uint4 *in, uint4 *out, long long nquads, Rows rows,
+                               int beside) {
+  begin_conversion(beside);
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < nquads;
        u += (long long)gridDim.x * blockDim.x) {
-    const uint4 w = in[u];
+    const uint4 w = in[rows.at(u)];
     const uint2 a = expand_packed4(w.x), b = expand_packed4(w.y), c = expand_packed4(w.z),
                 d = expand_packed4(w.w);
     out[2 * u] = make_uint4(a.x, a.y, b.x, b.y);
     out[2 * u + 1] = make_uint4(c.x, c.y, d.x, d.y);
   }
+  end_conversion(beside);
 }
 
 // xgpuSwizzleInput's layout (cpu_util.c:235-255) back to [t][f][s][p][c]:
@@ -178,12 +203,14 @@ __global__ void unpack4_kernel(const uint4 *in, uint4 *out, long long nquads) {
 // 4x4 with byte permutes, and writes one 4-byte word to each of the four
 // sample rows (consecutive threads write consecutive words of a row).
 __global__ void unswizzle_kernel(const uint4 *in, uint32_t *out, long long quads,
-                                 long long row_words) {
-  // quads = (t/4) * row_words; row_words = f*n (4 bytes per station)
+                                 long long row_words, long long pitch, int beside) {
+  begin_conversion(beside);
+  // quads = (t/4) * row_words; row_words = f*n (4 bytes per station); pitch: the
+  // same of the band
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < quads;
        u += (long long)gridDim.x * blockDim.x) {
     const long long tq = u / row_words, e4 = u - tq * row_words;
-    const uint4 w = in[u];
+    const uint4 w = in[tq * pitch + e4];
     const uint32_t lo01 = __byte_perm(w.x, w.y, 0x5140), hi01 = __byte_perm(w.x, w.y, 0x7362);
     const uint32_t lo23 = __byte_perm(w.z, w.w, 0x5140), hi23 = __byte_perm(w.z, w.w, 0x7362);
     uint32_t *o = out + 4 * tq * row_words + e4;
@@ -192,16 +219,19 @@ __global__ void unswizzle_kernel(const uint4 *in, uint32_t *out, long long quads
     o[2 * row_words] = __byte_perm(hi01, hi23, 0x5410);
     o[3 * row_words] = __byte_perm(hi01, hi23, 0x7632);
   }
+  end_conversion(beside);
 }
 
 // xGPU's COMPLEX_BLOCK_SIZE=32 input (read by omp_xengine.c:61-78,
 // shared_transfer_4.cuh:69-86) -> [t][f][s][p]{re,im}.  A 64-byte block holds
 // 16 consecutive (t,f,s) stations: {X.re,Y.re} pairs in bytes 0-31, {X.im,Y.im}
 // pairs in bytes 32-63.  One thread turns 4 stations (8 + 8 bytes) into 16.
-__global__ void unblock32_kernel(const uint2 *in, uint4 *out, long long quads) {
+__global__ void unblock32_kernel(const uint2 *in, uint4 *out, long long quads, Rows rows,
+                                 int beside) {
+  begin_conversion(beside);
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < quads;
        u += (long long)gridDim.x * blockDim.x) {
-    const long long blk = u >> 2;
+    const long long blk = rows.at(u >> 2);   // rows of whole blocks (n is a multiple of 16)
     const int q = (int)(u & 3);
     const uint2 re = in[blk * 8 + q];      // bytes 8q .. 8q+7 of the block
     const uint2 im = in[blk * 8 + 4 + q];  // bytes 32+8q ..
@@ -212,6 +242,7 @@ __global__ void unblock32_kernel(const uint2 *in, uint4 *out, long long quads) {
     o.w = __byte_perm(re.y, im.y, 0x7362);
     out[u] = o;
   }
+  end_conversion(beside);
 }
 
 // Seeded synthetic bytes; the same hash and tables as the host generator.
@@ -308,27 +339,44 @@ cudaError_t launch_format(const void *state, int state_is_float, const Sizes &s,
   return cudaLaunchKernelEx(&cfg, k, state, s.n, (int)s.nbaseline, f0, o);
 }
 
-cudaError_t launch_unpack4(const uint8_t *in, int8_t *out, long long nsamples, cudaStream_t st) {
-  const long long nquads = nsamples / 16;  // nsamples = 2*n*f*t, a multiple of 32 (n % 16 == 0)
-  fmt::unpack4_kernel<<<fmt::grid_for(nquads, 256), 256, 0, st>>>((const uint4 *)in,
-                                                                  (uint4 *)out, nquads);
-  return cudaGetLastError();
+// A programmatic launch of one of the conversions over `work` thread items.
+template <class... A>
+static cudaError_t launch_conversion(void (*kernel)(A...), long long work, cudaStream_t st,
+                                     A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(fmt::grid_for(work, 256));
+  cfg.blockDim = dim3(256);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-cudaError_t launch_unswizzle_dp4a(const int8_t *in, int8_t *out, const Sizes &s,
-                                  cudaStream_t st) {
-  const long long row_words = (long long)s.f * s.n;   // t is a multiple of 4 (ntimepipe % 16 == 0)
-  const long long quads = (long long)(s.t / 4) * row_words;
-  fmt::unswizzle_kernel<<<fmt::grid_for(quads, 256), 256, 0, st>>>((const uint4 *)in,
-                                                                   (uint32_t *)out, quads, row_words);
-  return cudaGetLastError();
+cudaError_t launch_unpack4(const uint8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
+                           bool beside) {
+  // 2n bytes a channel, n a multiple of 16
+  const long long row = (long long)s.f * s.n / 8, quads = row * s.t;
+  return launch_conversion(fmt::unpack4_kernel, quads, st, (const uint4 *)in, (uint4 *)out, quads,
+                           fmt::Rows{row, (long long)s.fin * s.n / 8}, (int)beside);
 }
 
-cudaError_t launch_unblock32(const int8_t *in, int8_t *out, long long nbytes, cudaStream_t st) {
-  const long long quads = nbytes / 16;
-  fmt::unblock32_kernel<<<fmt::grid_for(quads, 256), 256, 0, st>>>((const uint2 *)in,
-                                                                   (uint4 *)out, quads);
-  return cudaGetLastError();
+cudaError_t launch_unswizzle_dp4a(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
+                                  bool beside) {
+  const long long row = (long long)s.f * s.n;   // t is a multiple of 4 (ntimepipe % 16 == 0)
+  const long long quads = (long long)(s.t / 4) * row;
+  return launch_conversion(fmt::unswizzle_kernel, quads, st, (const uint4 *)in, (uint32_t *)out,
+                           quads, row, (long long)s.fin * s.n, (int)beside);
+}
+
+cudaError_t launch_unblock32(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
+                             bool beside) {
+  const long long row = (long long)s.f * s.n / 16;   // blocks of 16 stations
+  const long long quads = 4 * row * s.t;
+  return launch_conversion(fmt::unblock32_kernel, quads, st, (const uint2 *)in, (uint4 *)out, quads,
+                           fmt::Rows{row, (long long)s.fin * s.n / 16}, (int)beside);
 }
 
 void gauss_thresholds(double sigma, uint32_t thr[254]) {

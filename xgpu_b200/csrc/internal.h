@@ -27,6 +27,7 @@ enum DeviceError : int {
   kErrTimeoutDrain = 3,      // epilogue gave up waiting for the accumulator
   kErrTimeoutPanel = 4,      // plain engine gave up waiting for an input panel
   kErrTimeoutConvert = 5,    // packed-input converter gave up waiting for a loaded stage
+  kErrSharedBase = 6,        // dynamic shared memory not aligned to 1024 bytes
 };
 
 struct Sizes {
@@ -124,7 +125,9 @@ bool tc2_single_item(int tcount, const TcTuning &tune);
 // The setting for a call of a chain that overlap one another, with `before` calls
 // ahead of it (CTA pairs on part of the SMs, or the context's own); last: the
 // caller waits for it.
-TcTuning tc2_chain_tuning(const Sizes &s, const TcTuning &own, int before, bool last);
+TcTuning tc2_chain_tuning(const Sizes &s, const TcTuning &own, int before, bool last, bool packed);
+// Pipeline stages (of a 256x256 tile and 128 samples) of one call over all of s.
+long long tc2_stages(const Sizes &s);
 long long words_elems(const Sizes &s);
 // A dump's destination: matLength Complex as 32-bit words.
 struct DumpOut {
@@ -177,9 +180,16 @@ cudaError_t tc_configure_device();
 cudaError_t tc2_set_smem_attribute();
 
 // ---- input conversion, output formatting, synthetic input -----------------
-cudaError_t launch_unpack4(const uint8_t *in, int8_t *out, long long nsamples, cudaStream_t st);
-cudaError_t launch_unswizzle_dp4a(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st);
-cudaError_t launch_unblock32(const int8_t *in, int8_t *out, long long nbytes, cudaStream_t st);
+// `in` holds s.fin channels per row and points at the first that the context
+// correlates; `out` is compact.  Launched programmatically.  beside: the launch
+// before it on `st` is an engine launch that reads neither `in` (complete
+// already) nor `out`: the conversion runs beside it, and waits for it at its end.
+cudaError_t launch_unpack4(const uint8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
+                           bool beside);
+cudaError_t launch_unswizzle_dp4a(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
+                                  bool beside);
+cudaError_t launch_unblock32(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
+                             bool beside);
 // Channels [f0, f0 + fcount) of the buffer (int64 or float) into o.out in its
 // order and type (fcount < 0: through the last channel; other channels' words
 // are untouched).  Launched programmatically.  host_out: the output is mapped

@@ -71,20 +71,13 @@ struct Internal {
   void *d_in[2] = {nullptr, nullptr};  // one call's input, as supplied
   // Packed 4+4-bit (unless the CTA-pair kernel expands it itself:
   // packed_in_kernel), DP4A-swizzled and block-32 input is converted to int8
-  // [t][f][s][p][c] on its own stream into one of two buffers, so the
-  // conversion of call k+1 is queued without waiting for the engine of call
-  // k (measured: the two kernels seldom share the SMs, so a converted call
-  // costs its conversion plus its engine launch).
+  // [t][f][s][p][c] by a kernel ahead of the engine's, into one of two buffers:
+  // the conversion of call k+1 runs beside the engine launch of call k (whose
+  // CTAs leave it room on their SMs), which reads the other one.
   int8_t *d_conv[2] = {nullptr, nullptr};
-  cudaStream_t s_conv = nullptr;
-  cudaEvent_t conv_done[2] = {nullptr, nullptr};
-  cudaEvent_t conv_free[2] = {nullptr, nullptr};   // engine that read d_conv[k] finished
-  bool conv_used[2] = {false, false};
   int conv_cur = 0;
-  cudaEvent_t caller_ev = nullptr;                 // orders caller-stream work before a conversion
-  // A context of a channel range with a converted format gathers its channels
-  // of device-resident input here (on s_conv) before converting them.
-  void *d_slice = nullptr;
+  bool engine_tail = false;   // the last operation on s_own is an engine launch of this context
+  bool unpack = false;        // the call in hand converts packed input for the CTA-pair kernel
   void *d_state = nullptr;             // integration buffer
   // Launches of the CTA-pair kernel with short items put their sums into
   // this word buffer (one 64-bit word per visibility, im * 2^32 + re: half
@@ -213,15 +206,7 @@ int free_device(Internal *in) {
   }
   for (int k = 0; k < 2; ++k) {
     if (in->d_conv[k]) cudaFree(in->d_conv[k]);
-    if (in->conv_done[k]) cudaEventDestroy(in->conv_done[k]);
-    if (in->conv_free[k]) cudaEventDestroy(in->conv_free[k]);
   }
-  if (in->s_conv) {
-    cudaStreamSynchronize(in->s_conv);
-    cudaStreamDestroy(in->s_conv);
-  }
-  if (in->caller_ev) cudaEventDestroy(in->caller_ev);
-  if (in->d_slice) cudaFree(in->d_slice);
   if (in->d_state) cudaFree(in->d_state);
   if (in->d_words) cudaFree(in->d_words);
   if (in->d_out) cudaFree(in->d_out);
@@ -281,7 +266,23 @@ const CUtensorMap *tensor_map(Internal *in, const void *ptr, const Sizes &g, boo
 // pre-pass.
 bool packed_in_kernel(const Internal *in) {
   return in->cfg.input_format == XGPU_INPUT_PACKED4 && in->int_state &&
-         in->cfg.engine == XGPU_ENGINE_TENSOR && in->use.wide;
+         in->cfg.engine == XGPU_ENGINE_TENSOR && in->use.wide && !in->unpack;
+}
+
+// Whether a call over device input converts packed input ahead of the CTA-pair
+// kernel all the same.  The kernel's own expansion makes a stage take 1.35 times
+// as long; the conversion of a long call passes beside the call before it, on the
+// caller's stream it could not.  N=512, T=8192: with F=64 (147,456 stages) 8 calls
+// and their dump 14.5 to 13.1 ms, and one call alone 1.22 to 1.14 ms; with F=16
+// chains of 2, 4 and 16 calls 0.66 to 0.68, 1.26 to 1.25 and 4.80 to 4.08 ms, but
+// one alone 0.34 to 0.39.  Shorter calls overlap one another, which converted ones
+// do not (N=256, F=32, T=4096, 10,240 stages: 16 calls 1.43 against 1.61 ms).
+bool unpack_ahead(const Internal *in) {
+  if (in->cfg.input_format != XGPU_INPUT_PACKED4 || !in->int_state || !in->use.wide ||
+      in->s_comp != in->s_own)
+    return false;
+  const long long stages = tc2_stages(in->szc);
+  return stages >= 100000 || (stages >= 30000 && in->chain >= 2);
 }
 
 // The tensor engine's setting for a call over device input.  What xgpuTune chose
@@ -295,7 +296,8 @@ TcTuning call_tuning(const Internal *in, bool waited) {
   if (in->tuned || !in->int_state || in->cfg.engine != XGPU_ENGINE_TENSOR || in->chain == 0 ||
       !overlaps)
     return in->tune;
-  return tc2_chain_tuning(in->szc, in->tune, in->chain, waited);
+  return tc2_chain_tuning(in->szc, in->tune, in->chain, waited,
+                          in->cfg.input_format == XGPU_INPUT_PACKED4);
 }
 
 // Queue the engine over channels [f0, f0 + fcount) of int8 input x (packed
@@ -328,6 +330,7 @@ int fold_words(Internal *in, bool after_adding = false) {
   in->words_stale = !zero;
   in->words_samples = 0;
   in->adding_tail = false;
+  in->engine_tail = false;
   return XGPU_OK;
 }
 
@@ -404,11 +407,9 @@ int launch_engine(Internal *in, const int8_t *x, const Sizes &s, int f0, int fco
 
 // Queue the engine over one call's device input (any format) on s_comp.
 // input_ready, when given, is the event after which the input is complete
-// (the host-to-device copy); converted formats wait for it on s_conv.
+// (the host-to-device copy).
 // compact: d_input holds only this context's channels (the copy the host path
-// makes); otherwise it is the caller's full-band input, read in place (int8,
-// or packed input the CTA-pair kernel expands) or gathered into d_slice
-// before its conversion (the other formats).  allow_words: as launch_engine's.
+// makes); otherwise it is the caller's full-band input, read in place.  allow_words: as launch_engine's.
 int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool compact,
                bool allow_words = true) {
   const Sizes &s = in->sz;
@@ -422,35 +423,24 @@ int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool 
   const bool packed = packed_in_kernel(in);
   bool tail = in->adding_tail && in->s_comp == in->s_own && !input_ready &&
               (in->cfg.input_format == XGPU_INPUT_INT8 || packed);
+  const bool engine_tail = in->engine_tail;
   in->adding_tail = false;
+  in->engine_tail = false;
   if (in->cfg.input_format != XGPU_INPUT_INT8 && !packed) {
     conv = in->conv_cur;
     in->conv_cur ^= 1;
-    if (in->conv_used[conv]) XGPU_CHECK(cudaStreamWaitEvent(in->s_conv, in->conv_free[conv], 0));
-    if (input_ready) XGPU_CHECK(cudaStreamWaitEvent(in->s_conv, input_ready, 0));
-    if (in->s_comp != in->s_own) {
-      // The caller's stream may have produced the input: convert after it.
-      XGPU_CHECK(cudaEventRecord(in->caller_ev, in->s_comp));
-      XGPU_CHECK(cudaStreamWaitEvent(in->s_conv, in->caller_ev, 0));
-    }
-    const void *src = d_input;
-    if (ranged) {
-      // this context's channels of every row of the band, gathered in order
-      XGPU_CHECK(cudaMemcpy2DAsync(in->d_slice, (size_t)(s.f * s.chan_bytes),
-                                   (const char *)d_input + s.fin0 * s.chan_bytes,
-                                   (size_t)(s.fband * s.chan_bytes), (size_t)(s.f * s.chan_bytes),
-                                   (size_t)s.rows, cudaMemcpyDeviceToDevice, in->s_conv));
-      src = in->d_slice;
-    }
+    if (input_ready) XGPU_CHECK(cudaStreamWaitEvent(in->s_comp, input_ready, 0));
+    // On the context's own stream the caller's input is complete already; on a
+    // caller's stream the work before the call may still be making it.
+    const bool beside = engine_tail && !input_ready;
+    const Sizes &from = ranged ? s : in->szc;
+    const int8_t *src = x + (ranged ? s.fin0 * s.chan_bytes : 0);
     if (in->cfg.input_format == XGPU_INPUT_PACKED4)
-      XGPU_CHECK(launch_unpack4((const uint8_t *)src, in->d_conv[conv], s.vec_length, in->s_conv));
+      XGPU_CHECK(launch_unpack4((const uint8_t *)src, in->d_conv[conv], from, in->s_comp, beside));
     else if (in->cfg.input_format == XGPU_INPUT_BLOCK32)
-      XGPU_CHECK(launch_unblock32((const int8_t *)src, in->d_conv[conv], 2 * s.vec_length,
-                                  in->s_conv));
+      XGPU_CHECK(launch_unblock32(src, in->d_conv[conv], from, in->s_comp, beside));
     else
-      XGPU_CHECK(launch_unswizzle_dp4a((const int8_t *)src, in->d_conv[conv], in->szc, in->s_conv));
-    XGPU_CHECK(cudaEventRecord(in->conv_done[conv], in->s_conv));
-    XGPU_CHECK(cudaStreamWaitEvent(in->s_comp, in->conv_done[conv], 0));
+      XGPU_CHECK(launch_unswizzle_dp4a(src, in->d_conv[conv], from, in->s_comp, beside));
     x = in->d_conv[conv];
   } else {
     if (input_ready) XGPU_CHECK(cudaStreamWaitEvent(in->s_comp, input_ready, 0));
@@ -464,10 +454,7 @@ int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool 
   if (r != XGPU_OK) return r;
   if (in->int_state) in->adding_tail = tail && conv < 0;   // tensor or dp4a engine
   if (wrote_state) in->state_zero = false;   // otherwise the call went to the words
-  if (conv >= 0) {
-    XGPU_CHECK(cudaEventRecord(in->conv_free[conv], in->s_comp));
-    in->conv_used[conv] = true;
-  }
+  in->engine_tail = in->s_comp == in->s_own;
   return XGPU_OK;
 }
 
@@ -475,6 +462,7 @@ int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool 
 // launch's), then read and clear the device error word.
 int check_device_error(Internal *in, cudaStream_t st = nullptr) {
   in->adding_tail = false;
+  in->engine_tail = false;
   in->chain = 0;
   XGPU_CHECK(cudaStreamSynchronize(st ? st : in->s_comp));
   const int err = *(volatile int *)in->h_err;
@@ -819,8 +807,7 @@ int xgpuInitEx(XGPUContext *context, int device_flags, const XGPUConfig *cfg_in)
       cudaHostGetDevicePointer((void **)&in->d_err, in->h_err, 0) != cudaSuccess ||
       (cfg.input_format != XGPU_INPUT_INT8 &&
        (cudaMalloc(&in->d_conv[0], (size_t)(2 * s.vec_length + 255) / 256 * 256) != cudaSuccess ||
-        cudaMalloc(&in->d_conv[1], (size_t)(2 * s.vec_length + 255) / 256 * 256) != cudaSuccess ||
-        (s.fband != s.f && cudaMalloc(&in->d_slice, in_bytes) != cudaSuccess)))) {
+        cudaMalloc(&in->d_conv[1], (size_t)(2 * s.vec_length + 255) / 256 * 256) != cudaSuccess))) {
     cudaGetLastError();
     return fail(XGPU_OUT_OF_MEMORY);
   }
@@ -830,14 +817,10 @@ int xgpuInitEx(XGPUContext *context, int device_flags, const XGPUConfig *cfg_in)
   in->s_comp = in->s_own;
   for (int b = 0; b < 2; ++b) {
     if (cudaEventCreateWithFlags(&in->copy_done[b], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&in->comp_done[b], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&in->conv_done[b], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&in->conv_free[b], cudaEventDisableTiming) != cudaSuccess)
+        cudaEventCreateWithFlags(&in->comp_done[b], cudaEventDisableTiming) != cudaSuccess)
       return fail(XGPU_CUDA_ERROR);
   }
-  if (cudaStreamCreateWithFlags(&in->s_conv, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaStreamCreateWithFlags(&in->s_dump, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaEventCreateWithFlags(&in->caller_ev, cudaEventDisableTiming) != cudaSuccess)
+  if (cudaStreamCreateWithFlags(&in->s_dump, cudaStreamNonBlocking) != cudaSuccess)
     return fail(XGPU_CUDA_ERROR);
   for (int k = 0; k < kMaxGroups + 2; ++k) {
     if (cudaEventCreateWithFlags(&in->group_in[k], cudaEventDisableTiming) != cudaSuccess ||
@@ -1011,6 +994,7 @@ int xgpuCudaXengine(XGPUContext *context, int syncOp) {
   XGPU_CHECK(cudaSetDevice(in->device));
 
   in->use = in->tune;
+  in->unpack = false;
   in->chain = 0;
   const int b = in->cur;
   in->cur ^= 1;
@@ -1047,6 +1031,7 @@ int xgpuCudaXengineDevice(XGPUContext *context, const void *device_input, int sy
   if (syncOp < SYNCOP_NONE || syncOp > SYNCOP_SYNC_COMPUTE) return XGPU_INVALID_ARGUMENT;
   XGPU_CHECK(cudaSetDevice(in->device));
   in->use = call_tuning(in, syncOp != SYNCOP_NONE);
+  in->unpack = unpack_ahead(in);
   // A call that the host waits for, with none before it, goes to the int64 buffer
   // itself: the words' fold would follow at once (N=736, F=18, T=912, one call
   // and its dump: 3.18 ms with words, 3.08 without).
@@ -1098,6 +1083,7 @@ int xgpuSetComputeStream(XGPUContext *context, void *stream) {
   cudaStream_t next = stream ? (cudaStream_t)stream : in->s_own;
   if (next == in->s_comp) return XGPU_OK;
   in->adding_tail = false;
+  in->engine_tail = false;
   in->chain = 0;
   // Order the new stream after everything queued on the old one.
   cudaEvent_t ev;

@@ -217,6 +217,11 @@ __device__ __forceinline__ void queue_done(int *queue, int takers) {
   }
 }
 
+// Shared memory of an SM less what a CTA without any takes (1 KB): an engine CTA
+// (whose own 1 KB counts too) within it leaves room beside it for blocks that
+// convert the next call's input.
+constexpr int kSmemBeside = 228 * 1024 - 1024;
+
 constexpr int kEpiThreads = 128;   // four epilogue warps, one per TMEM lane quarter
 
 // Staging of drained sums: one 2 KB row per station of a 32-station block (32
