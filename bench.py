@@ -155,8 +155,7 @@ WORD_MAX_SAMPLES = 65535
 def word_folds(tuning, t, warmup, steps):
     """Launches of the library's fold kernel inside a timed run of `steps`
     calls after `warmup`: CTA-pair launches whose items take at most 8 stages
-    of 128 samples put their sums into a word buffer (the first call of the
-    integration stores its words, the others add), folded before it would
+    of 128 samples put their sums into a word buffer, folded before it would
     pass 65535 samples and once at the closing flush."""
     if not tuning or not tuning["pair"]:
         return 0

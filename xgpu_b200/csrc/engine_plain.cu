@@ -332,10 +332,10 @@ __global__ void __launch_bounds__(kThreads, 5) xengine_dp4a_kernel(const __grid_
 // autocorrelation adds 512 a sample; the blocks off the diagonal stay much
 // longer).  dp4a does 4 samples' products for two issue slots of the pipe that
 // takes 4 x 3 float operations otherwise: N=64, F=10, T=1024 from 117 us per
-// call to 42 us, N=256 from 353 us to 125 us.  The float phase works on both
+// call to 33, N=256 from 354 to 110.  The float phase works on both
 // column polarisations at once with packed float pairs: the float pipe's rate
 // is the same, but half the instructions leave issue slots for the operand
-// loads (sums past 2^24 throughout, N=64: 113 to 98 us; N=256: 354 to 288).
+// loads (sums past 2^24 throughout, N=64: 113 to 101 us; N=256: 354 to 285).
 constexpr int kTcF = 32;                         // samples per chunk of the float phase
 constexpr int kRawPanelF = kTcF * kRowBytes;     // 4 KiB
 constexpr int kFloatPanel = kTcF * kBlk;         // float4 entries: [sample][slot]
@@ -598,6 +598,7 @@ __device__ __forceinline__ void fp32_whole(const Params &p, uint8_t *dsm, uint32
     }
     if (!float_phase<8>(p, dsm, bar0 + 16, f, rb, cb, p.t0 + ch * kTcD, 0, sum)) return;
   }
+  tc::pdl_trigger();
 #pragma unroll
   for (int e = 0; e < 8; ++e)
     if (in_buffer(p, i0, j0, e)) *buffer_slot(p, f, i0, j0, e) = sum[e];
@@ -605,7 +606,7 @@ __device__ __forceinline__ void fp32_whole(const Params &p, uint8_t *dsm, uint32
 
 // ---- the call split over a cluster
 // A launch with few blocks (small arrays, few channels) leaves SMs idle, and
-// alone on its SM a block takes 2.6 us per 64 samples where the dp4a pipe
+// alone on its SM a block takes 2.0 us per 64 samples where the dp4a pipe
 // needs 1.0.  So a cluster of kPieces CTAs shares the block:
 //  * first each takes a piece of the call's samples, with exact int32 sums
 //    from zero, and the pieces' sums are added through distributed shared
@@ -617,9 +618,9 @@ __device__ __forceinline__ void fp32_whole(const Params &p, uint8_t *dsm, uint32
 //  * when the buffer's sums are past 2^24 already (checked first), or the bound
 //    does not hold at the end, the float phase over all samples, each CTA
 //    keeping 8 / kPieces of the eight parts of every thread's tile.
-// Per call in chains at N=64, F=10, T=1024: 41.6 us whole, 20.0 in four pieces;
-// at N=16, F=1, T=512: 22 and 8; with samples of sigma 120, past 2^24 from the
-// second call on, at N=64: 98 and 95.
+// Per call in chains at N=64, F=10, T=1024: 33 us whole, 18 in four pieces; at
+// N=16, F=1, T=512: 18 and 7; with samples of sigma 120, past 2^24 from the
+// second call on, at N=64: 101 and 88.
 struct SplitShared {
   int past;            // CTAs whose share of the buffer is past 2^24, or breaks the bound
   unsigned power[8];   // each piece's largest input power
@@ -791,12 +792,11 @@ __global__ void __launch_bounds__(kThreads, 5) xengine_fp32_kernel(const __grid_
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  // Programmatic launch: the prologue runs beside the previous kernel's end.  A
-  // grid that fills the SMs lets the next one in at once; a split one only when
-  // its sums are done, as CTAs that wait would unbalance the SMs for the grid
-  // after them (N=128 in two pieces: 64 against 45 us).
+  // Programmatic launch: the prologue runs beside the previous kernel's end.  The
+  // next grid is let in only when the sums are done: CTAs that come earlier wait on
+  // whichever SMs have room, and then run as unevenly as they came (N=256, F=6,
+  // T=2048: 194 us per call in chains against 136; N=128, F=20 101 against 72).
   tc::pdl_wait();
-  if (kPieces == 1) tc::pdl_trigger();
   if constexpr (kPieces > 1) {
     fp32_split<kPieces>(p, dsm, bar0, (SplitShared *)(dsm + kPanelsFp32 + 8 * kBarriersFp32), f,
                         rb, cb);
@@ -837,11 +837,11 @@ static int plain_splits(const Sizes &s, int fcount, int tcount, bool overlap) {
 
 // Pieces of an FP32 launch (fp32_split), for 32768 samples at most (a piece's
 // power stays below 2^30).  Eight or four while the CTAs still fit the SMs about
-// once (5.5 each: N=128, F=10, 200 blocks, runs 44 us with four pieces, 60
+// once (5.5 each: N=128, F=10, 200 blocks, runs 40 us with four pieces, 52
 // without); a piece of fewer than 256 samples (eight) or 128 (four) costs more
 // in the exchange than it gains, unless the SMs are nearly empty.  Two pieces
-// only there: at 288 blocks they gain nothing (N=256, F=4: 60 against 60 us) and
-// the float phase loses 12%.
+// only there: at 288 blocks they gain nothing (N=256, F=4: 55 against 52 us) and
+// the float phase loses 10%.
 static int fp32_pieces(const Sizes &s, int fcount, int tcount) {
   const int sms = current_device_sms();
   const dim3 g = plain_grid(s, fcount);

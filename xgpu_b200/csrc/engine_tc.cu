@@ -12,8 +12,9 @@
 // G is a plain int8 x int8 -> int32 GEMM with both operands "MN-major" (the
 // 4N input bytes of one sample are contiguous), so the kernel reads the input
 // exactly as it lies in HBM: no corner turn, no negation of -128, one
-// accumulator.  The two sums of each complex part are formed in int64 when
-// the accumulator is drained, so the result is exact.
+// accumulator.  The two sums of each complex part are formed in int32, which
+// holds them for the 32768 samples of a launch at most, when the accumulator is
+// drained, and added to int64, so the result is exact.
 //
 // Work items: (job, channel, time split, 128x128 tile of G on or below the
 // diagonal), a tile being 32 stations x 2 pols x re/im on each side.  A
@@ -26,8 +27,8 @@
 //             M=N=128, K=32, into one of two TMEM accumulators (2 x 128
 //             columns), so a tile's drain overlaps the next tile's MMAs
 //   warps 2-5 epilogue: drain TMEM (tcgen05.ld 32x32b), combine the re/im
-//             rows of every input with two warp shuffles into int64 (re, im)
-//             pairs staged in shared memory (one 2 KB row per station), then
+//             rows of every input with two warp shuffles into (re, im) pairs,
+//             widened to int64 and staged in shared memory (one 2 KB row per station), then
 //             32 lanes hand the rows to the bulk-copy engine: a plain bulk
 //             store when the item is the only writer of a zero buffer, a bulk
 //             reduce-add (cp.reduce.async.bulk .add.u64) otherwise -- the int64

@@ -2,8 +2,8 @@
 // tiles of the Gram matrix.
 //
 // Same arithmetic as engine_tc.cu (G = A A^T over the int8 input bytes of
-// each sample, MN-major operands straight from HBM, re/im combined in int64
-// when draining), with the tile doubled in both directions and shared by the
+// each sample, MN-major operands straight from HBM, re/im combined when
+// draining), with the tile doubled in both directions and shared by the
 // two SMs of a cluster:
 //   * the pair computes rows [256R, 256R+256) x columns [256C, 256C+256) of G
 //     (64 x 64 stations) for one channel, R >= C;

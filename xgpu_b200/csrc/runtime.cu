@@ -300,11 +300,6 @@ TcTuning call_tuning(const Internal *in, bool waited) {
                           in->cfg.input_format == XGPU_INPUT_PACKED4);
 }
 
-// Queue the engine over channels [f0, f0 + fcount) of int8 input x (packed
-// input when `packed`: packed_in_kernel) on s_comp, in time segments; the
-// first segment stores when the buffer is known to be zero.  x has geometry s
-// (in->szc for the context's compact buffers, in->sz for a full-band device
-// input read in place, x then pointing at the context's first channel).
 // Word buffers up to this size are left zero by a fold.  The first launch after
 // it then adds, and the second overlaps it, which a launch that stores its words
 // does not allow: N=256, F=10 (11.8 MB), 32 calls and a dump on 36 CTAs, 475 to
@@ -312,9 +307,9 @@ TcTuning call_tuning(const Internal *in, bool waited) {
 // gain (N=496, F=11, 49 MB: two calls and a dump 920 to 946 us).
 constexpr long long kZeroWords = (24 << 20) / 8;
 
-// Add the words into the int64 buffer, on s_comp after
-// everything queued there: before the buffer is read, and before the words
-// would hold more than kWordsMaxSamples samples.  after_adding: the last
+// Add the words into the int64 buffer, on s_comp after everything queued
+// there: before the buffer is read, and before the words would hold more than
+// kWordsMaxSamples samples.  after_adding: the last
 // launch on s_comp is an adding engine launch of this context, which the fold
 // may then start beside (it waits for it before touching memory).  The next
 // engine launch does not overlap the fold; it only starts its prologue early.
@@ -334,6 +329,11 @@ int fold_words(Internal *in, bool after_adding = false) {
   return XGPU_OK;
 }
 
+// Queue the engine over channels [f0, f0 + fcount) of int8 input x (packed
+// input when `packed`: packed_in_kernel) on s_comp, in time segments; the
+// first segment stores when the buffer is known to be zero.  x has geometry s
+// (in->szc for the context's compact buffers, in->sz for a full-band device
+// input read in place, x then pointing at the context's first channel).
 // *tail: in, the launch may overlap the adding launch before it; out, the
 // last launch queued only added.  allow_words: launches of the CTA-pair
 // kernel with short items may put their sums into the word buffer.  The first
@@ -409,7 +409,8 @@ int launch_engine(Internal *in, const int8_t *x, const Sizes &s, int f0, int fco
 // input_ready, when given, is the event after which the input is complete
 // (the host-to-device copy).
 // compact: d_input holds only this context's channels (the copy the host path
-// makes); otherwise it is the caller's full-band input, read in place.  allow_words: as launch_engine's.
+// makes); otherwise it is the caller's full-band input, read in place.
+// allow_words: as launch_engine's.
 int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool compact,
                bool allow_words = true) {
   const Sizes &s = in->sz;
