@@ -930,16 +930,25 @@ long long tc2_stages(const Sizes &s) {
 // half as long again.  Calls of fewer than 200
 // stages keep the context's default: the host queues them no faster than that
 // runs, and the fold before a dump is then lost (N=32, F=2, T=544: 110 us for 25
-// calls and a dump, 115 with pairs).
+// calls and a dump, 115 with pairs).  So do calls whose 256 x 256 tiles cover more
+// than 1.2 times what their 128 x 128 tiles would (1.4 where one tile is all): 32
+// calls and their dump at N=32, F=100, T=4096 401 us and 630 with pairs, six at
+// N=208, F=13, T=2752 311 and 348.  And where pairs are the default, calls that
+// give every pair more than 32 stages spread its start and end well enough (four
+// at N=528, F=7, T=2048 768 us, 811 on part of the SMs).
 TcTuning tc2_chain_tuning(const Sizes &s, const TcTuning &own, int before, bool last,
                           bool packed) {
   long long steps = tc2_stages(s);
-  if (steps < 200) return own;
+  const int pairs = current_device_sms() / 2, part = before < 3 ? before + 1 : 4;
+  const long long p = (4LL * s.n + 2 * tc2::kHalf - 1) / (2 * tc2::kHalf);
+  const long long q = (4LL * s.n + tc2::kHalf - 1) / tc2::kHalf;
+  if (steps < 200 || (own.wide ? steps > 32 * pairs
+                               : 40 * p * (p + 1) > (p > 1 ? 12 : 14) * q * (q + 1)))
+    return own;
   if (packed) steps += steps / 2;
   TcTuning t;
   t.wide = 1;
   t.stall = own.stall;
-  const int pairs = current_device_sms() / 2, part = before < 3 ? before + 1 : 4;
   const int each = last ? 32 : 128;
   long long k = (steps + each - 1) / each;
   if (k < pairs / part) k = pairs / part;
