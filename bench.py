@@ -694,7 +694,8 @@ def main():
         # The FP32 engine adds each sample's exact product pair with one
         # rounding, as xGPU's float engine does: 6 FP32 instructions (FMUL,
         # FFMA, FADD per component) per complex MAC of 8 operations, where the
-        # measured rate counts 4 FMAs.  Its instruction ceiling is 4/6 of it.
+        # measured rate counts 4 FMAs.  The float loop's instruction ceiling is 4/6
+        # of it; calls whose sums stay below 2^24 run on dp4a and may pass it.
         detail["plain_fp32_n256_frac_of_instruction_ceiling"] = (
             detail["plain_fp32_n256_tops"] / (detail["core_fp32_peak_tops_measured"] * 4 / 6))
         if rank == 0:
