@@ -1,7 +1,7 @@
 """Untuned contexts choose the tensor-core kernel per call: chains of calls over
 device input run CTA pairs on part of the SMs from the second call on.  Chains
 of every length up to eight, over shapes below and above the work where the rule
-takes over, with items that use the word buffer or not, word buffers small
+takes over, others whose tiles or whose size it leaves to the default, with items that use the word buffer or not, word buffers small
 enough to be left zero by a fold and larger ones, packed input that the chain's
 calls expand in the kernel and the first call converts, and integrations that
 are dumped, continued, or cleared with words pending: bit-exact sums."""
@@ -10,7 +10,8 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SHAPES = [(32, 3, 256), (128, 10, 1024), (176, 13, 1552), (256, 24, 256), (400, 5, 384)]
+SHAPES = [(32, 3, 256), (128, 10, 1024), (176, 13, 1552), (256, 24, 256), (400, 5, 384),
+          (80, 37, 400), (400, 30, 512)]
 
 
 @pytest.mark.parametrize("fmt", ["int8", "packed4"])
