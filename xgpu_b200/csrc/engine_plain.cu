@@ -857,7 +857,7 @@ static int fp32_pieces(const Sizes &s, int fcount, int tcount) {
 
 // The kernels' dynamic shared memory (45.2 KB each), allowed once per
 // device.
-static cudaError_t plain_configure_device() {
+cudaError_t plain_configure_device() {
   static std::atomic<unsigned long long> done{0};
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);

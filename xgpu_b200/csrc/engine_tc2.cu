@@ -998,7 +998,7 @@ cudaError_t tc2_set_smem_attribute() {
         cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, tc2::kSmemBytes);
     if (e != cudaSuccess) return e;
   }
-  return cudaSuccess;
+  return load_kernel((const void *)tc2::fold_words_kernel);
 }
 
 cudaError_t launch_tc2(const CUtensorMap &map, const Sizes &s, int t0, int tcount, int64_t *state,

@@ -160,6 +160,16 @@ __global__ void __launch_bounds__(kHostThreads)
   }
 }
 
+static auto pick_format(int state_is_float, bool tiles) {
+  return state_is_float ? (tiles ? format_kernel<true, true> : format_kernel<true, false>)
+                        : (tiles ? format_kernel<false, true> : format_kernel<false, false>);
+}
+static auto pick_format_host(int state_is_float, bool tiles) {
+  return state_is_float
+             ? (tiles ? format_host_kernel<true, true> : format_host_kernel<true, false>)
+             : (tiles ? format_host_kernel<false, true> : format_host_kernel<false, false>);
+}
+
 // Conversions are programmatic launches between two engine launches.  Beside the
 // engine launch before it a conversion touches neither that one's input nor its
 // sums, so it starts at once and only ends after it (one block's wait keeps the
@@ -324,19 +334,15 @@ cudaError_t launch_format(const void *state, int state_is_float, const Sizes &s,
         (s.mat_length / s.f * fcount / 2 + fmt::kHostThreads - 1) / fmt::kHostThreads;
     cfg.gridDim = dim3((unsigned)(blocks < fmt::kHostBlocks ? blocks : fmt::kHostBlocks));
     cfg.blockDim = dim3(fmt::kHostThreads);
-    auto *k = state_is_float
-                  ? (tiles ? fmt::format_host_kernel<true, true> : fmt::format_host_kernel<true, false>)
-                  : (tiles ? fmt::format_host_kernel<false, true>
-                           : fmt::format_host_kernel<false, false>);
-    return cudaLaunchKernelEx(&cfg, k, state, s.n, (int)s.nbaseline, f0, fcount, o);
+    return cudaLaunchKernelEx(&cfg, fmt::pick_format_host(state_is_float, tiles), state, s.n,
+                              (int)s.nbaseline, f0, fcount, o);
   }
   // about 16 blocks per SM in all, at least one per channel
   const int blocks = (int)((s.mat_length / s.f + 255) / 256);
   const int most = (148 * 16 + fcount - 1) / fcount;
   cfg.gridDim = dim3((unsigned)(blocks < most ? blocks : most), (unsigned)fcount);
-  auto *k = state_is_float ? (tiles ? fmt::format_kernel<true, true> : fmt::format_kernel<true, false>)
-                           : (tiles ? fmt::format_kernel<false, true> : fmt::format_kernel<false, false>);
-  return cudaLaunchKernelEx(&cfg, k, state, s.n, (int)s.nbaseline, f0, o);
+  return cudaLaunchKernelEx(&cfg, fmt::pick_format(state_is_float, tiles), state, s.n,
+                            (int)s.nbaseline, f0, o);
 }
 
 // A programmatic launch of one of the conversions over `work` thread items.
@@ -353,6 +359,22 @@ static cudaError_t launch_conversion(void (*kernel)(A...), long long work, cudaS
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+cudaError_t load_conversion(int input_format) {
+  switch (input_format) {
+    case XGPU_INPUT_PACKED4: return load_kernel((const void *)fmt::unpack4_kernel);
+    case XGPU_INPUT_DP4A_SWIZZLED: return load_kernel((const void *)fmt::unswizzle_kernel);
+    case XGPU_INPUT_BLOCK32: return load_kernel((const void *)fmt::unblock32_kernel);
+    default: return cudaSuccess;
+  }
+}
+
+cudaError_t load_format(int state_is_float, int order) {
+  const bool tiles = order == REGISTER_TILE_TRIANGULAR_ORDER;
+  const cudaError_t e = load_kernel((const void *)fmt::pick_format(state_is_float, tiles));
+  return e != cudaSuccess ? e
+                          : load_kernel((const void *)fmt::pick_format_host(state_is_float, tiles));
 }
 
 cudaError_t launch_unpack4(const uint8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,

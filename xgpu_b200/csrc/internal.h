@@ -171,6 +171,15 @@ int make_panel_map(CUtensorMap *map, const void *dev_in, const Sizes &s, int row
 int make_packed_map(CUtensorMap *map, const void *dev_in, const Sizes &s);
 // 0 if the tensor-core kernel image loads on the current device.
 cudaError_t tc_check_device();
+// Loads a kernel on the current device.  CUDA otherwise loads it at its first
+// launch, which holds up what is queued around it: the fold behind a program's
+// first 20 calls of N=256, F=10, T=1024 took 0.3 to 2.4 ms to load where the
+// calls take 0.17.  Creating a context loads what its calls, dumps and flushes
+// launch.
+inline cudaError_t load_kernel(const void *kernel) {
+  cudaFuncAttributes a;
+  return cudaFuncGetAttributes(&a, kernel);
+}
 // Per-device set-up and facts, cached for devices 0 .. kDeviceCache-1 (others are
 // queried or set on every call): the SM count of the current device, and the
 // dynamic shared-memory allowance of both tcgen05 kernels on it.
@@ -178,6 +187,7 @@ constexpr int kDeviceCache = 64;
 int current_device_sms();
 cudaError_t tc_configure_device();
 cudaError_t tc2_set_smem_attribute();
+cudaError_t plain_configure_device();
 
 // ---- input conversion, output formatting, synthetic input -----------------
 // `in` holds s.fin channels per row and points at the first that the context
@@ -196,6 +206,10 @@ cudaError_t launch_unblock32(const int8_t *in, int8_t *out, const Sizes &s, cuda
 // host memory.
 cudaError_t launch_format(const void *state, int state_is_float, const Sizes &s, const DumpOut &o,
                           cudaStream_t st, int f0 = 0, int fcount = -1, bool host_out = false);
+// Load the kernels that the conversions and launch_format launch for a context's input format, and for
+// its buffer's type and its matrix order.
+cudaError_t load_conversion(int input_format);
+cudaError_t load_format(int state_is_float, int order);
 cudaError_t launch_generate(void *out, size_t nbytes, int kind, unsigned long long seed,
                             double sigma, cudaStream_t st);
 

@@ -796,6 +796,12 @@ int xgpuInitEx(XGPUContext *context, int device_flags, const XGPUConfig *cfg_in)
     fprintf(stderr, "xgpu: the tensor-core engine needs an sm_100 (B200-class) device\n");
     return fail(XGPU_CUDA_ERROR);
   }
+  if ((cfg.engine == XGPU_ENGINE_PLAIN && plain_configure_device() != cudaSuccess) ||
+      load_conversion((int)cfg.input_format) != cudaSuccess ||
+      load_format(in->int_state ? 0 : 1, (int)cfg.matrix_order) != cudaSuccess) {
+    cudaGetLastError();
+    return fail(XGPU_CUDA_ERROR);
+  }
 
   const Sizes &s = in->sz;
   const size_t in_bytes = (size_t)((s.input_bytes + 255) / 256 * 256);

@@ -244,6 +244,7 @@ extern "C" int xgpuServeRun(const XGPUServeJob *jobs, int njobs, const XGPUServe
     cudaGetLastError();
     return XGPU_CUDA_ERROR;
   }
+  SCHECK(load_format(0, TRIANGULAR_ORDER));
   if (!dev.init(opt.device_budget_bytes, true)) return XGPU_OUT_OF_MEMORY;
   if (!host.init(opt.host_budget_bytes ? opt.host_budget_bytes : ((size_t)8 << 30), false))
     return XGPU_OUT_OF_MEMORY;
