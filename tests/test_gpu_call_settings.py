@@ -1,0 +1,77 @@
+"""The kernel and grid of a call over device input, read from the launches that
+a profiler records (in a process of its own).  An untuned context runs CTA pairs
+on part of the SMs only for calls that the calls before them can overlap: not
+for a call whose predecessors have finished, however the program waited for
+them."""
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SCRIPT = r"""
+import json, os, tempfile, time
+import torch
+from torch.profiler import profile, ProfilerActivity
+import xgpu_b200 as xg
+
+def recorded(f):
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        f()
+        torch.cuda.synchronize()
+    path = os.path.join(tempfile.mkdtemp(), "trace.json")
+    p.export_chrome_trace(path)
+    with open(path) as fh:
+        ev = [e for e in json.load(fh)["traceEvents"] if e.get("cat") == "kernel"]
+    ev.sort(key=lambda e: e["ts"])
+    return [[e["name"].split("(")[0].split("::")[-1], e["args"]["grid"][0]] for e in ev]
+
+def context(n, f, t):
+    c = xg.Correlator(n, f, t, flags=xg.XGPU_DONT_REGISTER)
+    x = torch.randint(-8, 8, (4 * n * f * t,), device="cuda", dtype=torch.int8)
+    torch.cuda.synchronize()
+    return c, x
+
+def calls(c, x, k, sync=xg.SYNCOP_NONE, wait=None):
+    for _ in range(k):
+        c.run_device(x.data_ptr(), sync)
+        if wait:
+            wait()
+
+out = {}
+c, x = context(256, 10, 8192)      # a call takes about 0.1 ms
+recorded(lambda: calls(c, x, 1))
+c.clear()
+out["lone"] = recorded(lambda: calls(c, x, 1))
+c.clear()
+out["chain"] = recorded(lambda: calls(c, x, 6))
+c.clear()
+out["waited"] = recorded(lambda: calls(c, x, 6, wait=torch.cuda.synchronize))
+c.clear()
+out["slow"] = recorded(lambda: calls(c, x, 6, wait=lambda: time.sleep(0.005)))
+c.close()
+print(json.dumps(out))
+"""
+
+
+@pytest.fixture(scope="module")
+def launches(xg):
+    root = os.path.dirname(os.path.dirname(os.path.abspath(xg.__file__)))
+    r = subprocess.run([sys.executable, "-c", SCRIPT], cwd=root, capture_output=True, text=True,
+                       timeout=300)
+    assert r.returncode == 0, r.stderr[-2000:]
+    return json.loads(r.stdout.splitlines()[-1])
+
+
+def test_chain_runs_pairs_on_part_of_the_sms(launches):
+    assert len(launches["chain"]) == 6
+    assert launches["chain"][0] == launches["lone"][0]
+    assert all("tc2" in name and grid < 148 for name, grid in launches["chain"][1:])
+
+
+@pytest.mark.parametrize("how", ["waited", "slow"])
+def test_call_after_finished_calls_has_the_gpu(launches, how):
+    assert launches[how] == 6 * launches["lone"]

@@ -1,0 +1,59 @@
+"""Conversions beside engine launches where the order rests on the launch before
+the last one: calls of several launches (more than 32768 samples), whose later
+launches let the next conversion start at once, and calls over host and device
+input in turn, which share the two conversion buffers.  Every call's input
+differs; sums are bit-exact."""
+import numpy as np
+import pytest
+
+from test_gpu_conversions import encode
+
+pytestmark = pytest.mark.gpu
+
+
+def inputs(oracle_mod, fmt, n, f, t, count, seed):
+    import torch
+    host, dev, sums = [], [], []
+    for q in range(count):
+        b, x = encode(oracle_mod, fmt, n, f, t, seed + q)
+        host.append(np.ascontiguousarray(b).view(np.int8))
+        dev.append(torch.from_numpy(host[-1]).cuda())
+        sums.append(oracle_mod.xengine_i64(x, n, f, t))
+    torch.cuda.synchronize()
+    return host, dev, sums
+
+
+@pytest.mark.parametrize("fmt", ["packed4", "dp4a_swizzled", "block32"])
+@pytest.mark.parametrize("engine,grid", [("tensor", 0), ("tensor", 4), ("plain", 0)])
+def test_calls_of_several_launches(xg, oracle_mod, fmt, engine, grid):
+    n, f, t = 32, 2, 65536 + 256
+    host, dev, sums = inputs(oracle_mod, fmt, n, f, t, 4, 300)
+    with xg.Correlator(n, f, t, ntimepipe=16, engine=engine, input_format=fmt) as c:
+        if engine == "tensor":
+            c.tune(1, grid, 0)
+        for _ in range(2):
+            for d in dev:
+                c.run_device(d.data_ptr())
+        assert np.array_equal(c.dump_int64(), 2 * sum(sums))
+
+
+@pytest.mark.parametrize("fmt", ["packed4", "dp4a_swizzled", "block32"])
+@pytest.mark.parametrize("engine", ["tensor", "plain"])
+@pytest.mark.parametrize("sync", ["SYNCOP_NONE", "SYNCOP_SYNC_TRANSFER"])
+def test_host_and_device_calls_in_turn(xg, oracle_mod, fmt, engine, sync):
+    n, f, t = 96, 3, 1024
+    host, dev, sums = inputs(oracle_mod, fmt, n, f, t, 5, 400)
+    with xg.Correlator(n, f, t, ntimepipe=16, engine=engine, input_format=fmt) as c:
+        want = np.zeros_like(sums[0])
+        for q in range(15):
+            if q % 3 == 1:
+                # the host buffer may be refilled once the transfer before is done
+                c.set_input(host[q % 5])
+                c.run(getattr(xg, sync))
+                if sync == "SYNCOP_NONE":
+                    c.run_device(dev[(q + 1) % 5].data_ptr(), xg.SYNCOP_SYNC_TRANSFER)
+                    want += sums[(q + 1) % 5]
+            else:
+                c.run_device(dev[q % 5].data_ptr())
+            want += sums[q % 5]
+        assert np.array_equal(c.dump_int64(), want)

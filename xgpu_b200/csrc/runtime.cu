@@ -285,19 +285,38 @@ bool unpack_ahead(const Internal *in) {
   return stages >= 100000 || (stages >= 30000 && in->chain >= 2);
 }
 
+// Whether everything queued on the context's own stream has finished.  Relaxed, so
+// that a capture that this thread has begun on another stream stays valid.
+bool own_stream_idle(const Internal *in) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  const cudaError_t e = cudaStreamQuery(in->s_own);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e == cudaErrorNotReady) cudaGetLastError();   // not an error of the call in hand
+  return e == cudaSuccess;
+}
+
 // The tensor engine's setting for a call over device input.  What xgpuTune chose
 // holds for every call.  Otherwise a call that follows others the host has not
 // waited for is one of a chain, which CTA pairs on part of the SMs run faster
 // where the calls may overlap (tc2_chain_tuning); the first one, which may stay
-// alone, uses the context's default.
-TcTuning call_tuning(const Internal *in, bool waited) {
+// alone, uses the context's default.  So does a call that finds the ones before it
+// finished, by whichever way the program waited for them or because it is slower
+// than the GPU: nothing would run beside it on the other SMs (N=256, F=10, T=1024,
+// calls waited for one by one: 39 us on a quarter of the SMs, 27 on all).  A
+// setting for every SM needs no overlap.
+TcTuning call_tuning(Internal *in, bool waited) {
   const bool overlaps = in->s_comp == in->s_own && (in->cfg.input_format == XGPU_INPUT_INT8 ||
                                                     in->cfg.input_format == XGPU_INPUT_PACKED4);
   if (in->tuned || !in->int_state || in->cfg.engine != XGPU_ENGINE_TENSOR || in->chain == 0 ||
       !overlaps)
     return in->tune;
-  return tc2_chain_tuning(in->szc, in->tune, in->chain, waited,
-                          in->cfg.input_format == XGPU_INPUT_PACKED4);
+  const TcTuning t = tc2_chain_tuning(in->szc, in->tune, in->chain, waited,
+                                      in->cfg.input_format == XGPU_INPUT_PACKED4);
+  const bool part = t.grid > 0 && t.grid < current_device_sms() / 2 * 2;
+  if (!part || !own_stream_idle(in)) return t;
+  in->chain = 0;
+  return in->tune;
 }
 
 // Word buffers up to this size are left zero by a fold.  The first launch after
