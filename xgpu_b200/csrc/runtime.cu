@@ -113,6 +113,7 @@ struct Internal {
   // Calls over device input queued on the context's own stream since the host
   // last waited for it, or cleared or dumped the integration.
   int chain = 0;
+  int chain_before = 2;   // length of the chain before it (at first: more than one call)
   // The last operation queued on s_comp is an engine launch that only added
   // into the integration buffer (no store), on the context's own stream: the
   // next accumulating launch over other input may overlap it.
@@ -269,20 +270,9 @@ bool packed_in_kernel(const Internal *in) {
          in->cfg.engine == XGPU_ENGINE_TENSOR && in->use.wide && !in->unpack;
 }
 
-// Whether a call over device input converts packed input ahead of the CTA-pair
-// kernel all the same.  The kernel's own expansion makes a stage take 1.35 times
-// as long; the conversion of a long call passes beside the call before it, on the
-// caller's stream it could not.  N=512, T=8192: with F=64 (147,456 stages) 8 calls
-// and their dump 14.5 to 13.1 ms, and one call alone 1.22 to 1.14 ms; with F=16
-// chains of 2, 4 and 16 calls 0.66 to 0.68, 1.26 to 1.25 and 4.80 to 4.08 ms, but
-// one alone 0.34 to 0.39.  Shorter calls overlap one another, which converted ones
-// do not (N=256, F=32, T=4096, 10,240 stages: 16 calls 1.43 against 1.61 ms).
-bool unpack_ahead(const Internal *in) {
-  if (in->cfg.input_format != XGPU_INPUT_PACKED4 || !in->int_state || !in->use.wide ||
-      in->s_comp != in->s_own)
-    return false;
-  const long long stages = tc2_stages(in->szc);
-  return stages >= 100000 || (stages >= 30000 && in->chain >= 2);
+void end_chain(Internal *in) {
+  if (in->chain > 0) in->chain_before = in->chain;
+  in->chain = 0;
 }
 
 // Whether everything queued on the context's own stream has finished.  Relaxed, so
@@ -315,8 +305,31 @@ TcTuning call_tuning(Internal *in, bool waited) {
                                       in->cfg.input_format == XGPU_INPUT_PACKED4);
   const bool part = t.grid > 0 && t.grid < current_device_sms() / 2 * 2;
   if (!part || !own_stream_idle(in)) return t;
-  in->chain = 0;
+  end_chain(in);
   return in->tune;
+}
+
+// Whether a call over device input converts packed input ahead of the CTA-pair
+// kernel all the same.  The kernel's own expansion makes a stage take 1.35 times
+// as long; the conversion of a long call passes beside the call before it, on the
+// caller's stream it could not.  Shorter calls overlap one another, which converted
+// ones do not (N=256, F=32, T=4096, 10,240 stages: 16 calls 1.43 against 1.61 ms).
+// Chains with their dump, N=512, T=8192, F=64 (147,456 stages): 8 calls 14.7 to 13.2
+// ms; F=16 (36,864): 4 and 8 calls 2.59 to 2.46 and 3.79 to 3.44; N=768, F=16
+// (79,872) 8.17 to 7.34, N=384, F=24, T=6144 (24,192) no gain.  Under the power cap,
+// after seconds without a pause, it draws the clock down and gives less: chains of
+// 16 at N=512, F=64 1.21 to 1.19 ms a call, F=16 306 to 296 us, of 4 at F=64 1.21 to
+// 1.23, F=256 4.87 to 4.91.  A call by itself only has it to pay for then (N=512,
+// F=64 1.25 to 1.34 ms, F=24 486 to 509 us), so calls that find nothing before
+// them, or came one by one last time, expand in the kernel.
+bool unpack_ahead(Internal *in) {
+  if (in->cfg.input_format != XGPU_INPUT_PACKED4 || !in->int_state || !in->use.wide ||
+      in->s_comp != in->s_own)
+    return false;
+  const long long stages = tc2_stages(in->szc);
+  if (stages < 30000) return false;
+  if (in->chain > 0 && own_stream_idle(in)) end_chain(in);
+  return stages >= 100000 ? in->chain > 0 || in->chain_before > 1 : in->chain >= 2;
 }
 
 // Word buffers up to this size are left zero by a fold.  The first launch after
@@ -483,7 +496,7 @@ int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool 
 int check_device_error(Internal *in, cudaStream_t st = nullptr) {
   in->adding_tail = false;
   in->engine_tail = false;
-  in->chain = 0;
+  end_chain(in);
   XGPU_CHECK(cudaStreamSynchronize(st ? st : in->s_comp));
   const int err = *(volatile int *)in->h_err;
   if (err != 0) {
@@ -902,7 +915,7 @@ int xgpuClearDeviceIntegrationBuffer(XGPUContext *context) {
     in->words_samples = 0;
   }
   in->adding_tail = false;
-  in->chain = 0;
+  end_chain(in);
   in->state_zero = true;
   return XGPU_OK;
 }
@@ -1021,7 +1034,7 @@ int xgpuCudaXengine(XGPUContext *context, int syncOp) {
 
   in->use = in->tune;
   in->unpack = false;
-  in->chain = 0;
+  end_chain(in);
   const int b = in->cur;
   in->cur ^= 1;
   if (syncOp == SYNCOP_DUMP) {
@@ -1110,7 +1123,7 @@ int xgpuSetComputeStream(XGPUContext *context, void *stream) {
   if (next == in->s_comp) return XGPU_OK;
   in->adding_tail = false;
   in->engine_tail = false;
-  in->chain = 0;
+  end_chain(in);
   // Order the new stream after everything queued on the old one.
   cudaEvent_t ev;
   XGPU_CHECK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
