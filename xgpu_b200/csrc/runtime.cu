@@ -112,7 +112,8 @@ struct Internal {
   TcTuning use;         // the setting of the call in hand (call_tuning)
   // Calls over device input queued on the context's own stream since the host
   // last waited for it, or cleared or dumped the integration.
-  int chain = 0;
+  int chain = 0;          // up to kLongChain
+  static constexpr int kLongChain = 1000;
   int chain_before = 2;   // length of the chain before it (at first: more than one call)
   // The last operation queued on s_comp is an engine launch that only added
   // into the integration buffer (no store), on the context's own stream: the
@@ -1077,7 +1078,7 @@ int xgpuCudaXengineDevice(XGPUContext *context, const void *device_input, int sy
   const bool words = syncOp == SYNCOP_NONE || in->chain > 0 || in->words_dirty;
   int r = run_engine(in, device_input, nullptr, false, words);
   if (r != XGPU_OK) return r;
-  ++in->chain;
+  if (in->chain < Internal::kLongChain) ++in->chain;
   return finish_call(context, in, syncOp);
 }
 
