@@ -304,7 +304,11 @@ int xgpuSetComputeStream(XGPUContext *context, void *stream);
  * context.  On its own stream a context lets an accumulating call over
  * device-resident input start while the previous call's launch finishes (the
  * two only add into the integration), so callers that time or order work
- * should record their events on this stream rather than switch streams. */
+ * should record their events on this stream rather than switch streams.  Work
+ * that a caller queues between calls (an event that takes a time, a copy, a
+ * kernel) ends that overlap, so a context whose own stream has been handed out no
+ * longer chooses settings that rest on it (see xgpuTuning); those that xgpuTune
+ * chose it keeps. */
 void *xgpuComputeStream(XGPUContext *context);
 
 /* Extension with no counterpart in the reference: correlate once without

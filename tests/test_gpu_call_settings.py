@@ -2,7 +2,8 @@
 a profiler records (in a process of its own).  An untuned context runs CTA pairs
 on part of the SMs only for calls that the calls before them can overlap: not
 for a call whose predecessors have finished, however the program waited for
-them."""
+them, and not once the program holds the stream and may queue its own work
+between the calls."""
 import json
 import os
 import subprocess
@@ -52,6 +53,9 @@ c.clear()
 out["waited"] = recorded(lambda: calls(c, x, 6, wait=torch.cuda.synchronize))
 c.clear()
 out["slow"] = recorded(lambda: calls(c, x, 6, wait=lambda: time.sleep(0.005)))
+c.clear()
+c.stream
+out["stream held"] = recorded(lambda: calls(c, x, 6))
 c.close()
 c, x = context(512, 48, 8192, "packed4")    # 110,592 pipeline stages, 0.9 ms a call
 for how, sync, wait in (("api", xg.SYNCOP_SYNC_COMPUTE, None),
@@ -84,6 +88,10 @@ def test_chain_runs_pairs_on_part_of_the_sms(launches):
 @pytest.mark.parametrize("how", ["waited", "slow"])
 def test_call_after_finished_calls_has_the_gpu(launches, how):
     assert launches[how] == 6 * launches["lone"]
+
+
+def test_held_stream_keeps_the_default(launches):
+    assert launches["stream held"] == 6 * launches["lone"]
 
 
 @pytest.mark.parametrize("how", ["api", "device"])

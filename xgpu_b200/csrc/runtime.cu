@@ -115,6 +115,7 @@ struct Internal {
   int chain = 0;          // up to kLongChain
   static constexpr int kLongChain = 1000;
   int chain_before = 2;   // length of the chain before it (at first: more than one call)
+  bool stream_given = false;   // the program has s_own's handle
   // The last operation queued on s_comp is an engine launch that only added
   // into the integration buffer (no store), on the context's own stream: the
   // next accumulating launch over other input may overlap it.
@@ -294,8 +295,11 @@ bool own_stream_idle(const Internal *in) {
 // alone, uses the context's default.  So does a call that finds the ones before it
 // finished, by whichever way the program waited for them or because it is slower
 // than the GPU: nothing would run beside it on the other SMs (N=256, F=10, T=1024,
-// calls waited for one by one: 39 us on a quarter of the SMs, 27 on all).  A
-// setting for every SM needs no overlap.
+// calls waited for one by one: 39 us on a quarter of the SMs, 27 on all).  And so
+// do the calls of a program that has the stream's handle (xgpuComputeStream) and may
+// queue work of its own between them: behind a timed event, say, no call overlaps
+// the one before (64 calls, each with one: 31 us a call on a quarter of the SMs, 20
+// on all).  A setting for every SM needs no overlap.
 TcTuning call_tuning(Internal *in, bool waited) {
   const bool overlaps = in->s_comp == in->s_own && (in->cfg.input_format == XGPU_INPUT_INT8 ||
                                                     in->cfg.input_format == XGPU_INPUT_PACKED4);
@@ -305,7 +309,9 @@ TcTuning call_tuning(Internal *in, bool waited) {
   const TcTuning t = tc2_chain_tuning(in->szc, in->tune, in->chain, waited,
                                       in->cfg.input_format == XGPU_INPUT_PACKED4);
   const bool part = t.grid > 0 && t.grid < current_device_sms() / 2 * 2;
-  if (!part || !own_stream_idle(in)) return t;
+  if (!part) return t;
+  if (in->stream_given) return in->tune;
+  if (!own_stream_idle(in)) return t;
   end_chain(in);
   return in->tune;
 }
@@ -1137,7 +1143,9 @@ int xgpuSetComputeStream(XGPUContext *context, void *stream) {
 
 void *xgpuComputeStream(XGPUContext *context) {
   Internal *in = get(context);
-  return in ? (void *)in->s_comp : nullptr;
+  if (!in) return nullptr;
+  if (in->s_comp == in->s_own) in->stream_given = true;
+  return (void *)in->s_comp;
 }
 
 int xgpuTune(XGPUContext *context, int ksplit, int grid, int pair) {
