@@ -43,12 +43,14 @@ def calls(c, x, k, sync=xg.SYNCOP_NONE, wait=None):
             wait()
 
 out = {}
-c, x = context(256, 10, 8192)      # a call takes about 0.1 ms
+c, x = context(256, 10, 32768)     # a call takes about 0.3 ms
 recorded(lambda: calls(c, x, 1))
 c.clear()
 out["lone"] = recorded(lambda: calls(c, x, 1))
 c.clear()
 out["chain"] = recorded(lambda: calls(c, x, 6))
+c.clear()
+out["transfer"] = recorded(lambda: calls(c, x, 6, xg.SYNCOP_SYNC_TRANSFER))
 c.clear()
 out["waited"] = recorded(lambda: calls(c, x, 6, wait=torch.cuda.synchronize))
 c.clear()
@@ -66,6 +68,11 @@ calls(c, x, 3)
 torch.cuda.synchronize()
 out["packed chain"] = recorded(lambda: calls(c, x, 4))
 c.close()
+for name, sync in (("first", xg.SYNCOP_NONE), ("first transfer", xg.SYNCOP_SYNC_TRANSFER),
+                   ("first waited", xg.SYNCOP_SYNC_COMPUTE)):
+    c, x = context(400, 5, 384)    # short items: a call that may be one of many uses the words
+    out[name] = recorded(lambda: (calls(c, x, 1, sync), c.flush()))
+    c.close()
 print(json.dumps(out))
 """
 
@@ -92,6 +99,14 @@ def test_call_after_finished_calls_has_the_gpu(launches, how):
 
 def test_held_stream_keeps_the_default(launches):
     assert launches["stream held"] == 6 * launches["lone"]
+
+
+def test_transfer_sync_waits_for_no_engine(launches):
+    """SYNCOP_SYNC_TRANSFER returns with the engine at work (device input has no
+    transfer), so its calls are a chain's like any others."""
+    assert launches["transfer"] == launches["chain"]
+    assert launches["first transfer"] == launches["first"]
+    assert launches["first waited"] != launches["first"]
 
 
 @pytest.mark.parametrize("how", ["api", "device"])

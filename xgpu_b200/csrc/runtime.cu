@@ -1076,12 +1076,14 @@ int xgpuCudaXengineDevice(XGPUContext *context, const void *device_input, int sy
   if (!device_input || ((uintptr_t)device_input & 15) != 0) return XGPU_INVALID_ARGUMENT;
   if (syncOp < SYNCOP_NONE || syncOp > SYNCOP_SYNC_COMPUTE) return XGPU_INVALID_ARGUMENT;
   XGPU_CHECK(cudaSetDevice(in->device));
-  in->use = call_tuning(in, syncOp != SYNCOP_NONE);
+  // SYNCOP_SYNC_TRANSFER has no transfer to wait for here, and waits for no engine.
+  const bool waited = syncOp == SYNCOP_DUMP || syncOp == SYNCOP_SYNC_COMPUTE;
+  in->use = call_tuning(in, waited);
   in->unpack = unpack_ahead(in);
   // A call that the host waits for, with none before it, goes to the int64 buffer
   // itself: the words' fold would follow at once (N=736, F=18, T=912, one call
   // and its dump: 3.18 ms with words, 3.08 without).
-  const bool words = syncOp == SYNCOP_NONE || in->chain > 0 || in->words_dirty;
+  const bool words = !waited || in->chain > 0 || in->words_dirty;
   int r = run_engine(in, device_input, nullptr, false, words);
   if (r != XGPU_OK) return r;
   if (in->chain < Internal::kLongChain) ++in->chain;
