@@ -42,15 +42,22 @@ def calls(c, x, k, sync=xg.SYNCOP_NONE, wait=None):
         if wait:
             wait()
 
+def chain(c, x, sync=xg.SYNCOP_NONE):
+    # of three, the one least interrupted on the host: a call that the host queues
+    # late finds the ones before it finished
+    runs = []
+    for _ in range(3):
+        c.clear()
+        runs.append(recorded(lambda: calls(c, x, 6, sync)))
+    return min(runs, key=lambda r: sum(grid for name, grid in r))
+
 out = {}
-c, x = context(256, 10, 32768)     # a call takes about 0.3 ms
+c, x = context(256, 10, 8192)      # a call takes about 0.1 ms
 recorded(lambda: calls(c, x, 1))
 c.clear()
 out["lone"] = recorded(lambda: calls(c, x, 1))
-c.clear()
-out["chain"] = recorded(lambda: calls(c, x, 6))
-c.clear()
-out["transfer"] = recorded(lambda: calls(c, x, 6, xg.SYNCOP_SYNC_TRANSFER))
+out["chain"] = chain(c, x)
+out["transfer"] = chain(c, x, xg.SYNCOP_SYNC_TRANSFER)
 c.clear()
 out["waited"] = recorded(lambda: calls(c, x, 6, wait=torch.cuda.synchronize))
 c.clear()
