@@ -57,3 +57,33 @@ def test_host_and_device_calls_in_turn(xg, oracle_mod, fmt, engine, sync):
                 c.run_device(dev[q % 5].data_ptr())
             want += sums[q % 5]
         assert np.array_equal(c.dump_int64(), want)
+
+
+@pytest.mark.parametrize("band,off", [(0, 0), (18, 1)])
+def test_long_calls_on_a_callers_stream(xg, band, off):
+    """134 MB of int8 samples a call, converted with nothing beside: launched plainly.
+    Every format gives the sums of the same samples as int8."""
+    import torch
+    n, f, t = 512, 16, 4096
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    xs = [torch.randint(-8, 8, (t, (band or f) * n * 2, 2), generator=gen, device="cuda",
+                        dtype=torch.int8) for _ in range(2)]
+    encoded = {
+        "int8": lambda x: x,
+        "packed4": lambda x: (x[..., 0] << 4) | (x[..., 1] & 15),
+        "dp4a_swizzled": lambda x: x.view(t // 4, 4, -1).transpose(1, 2),
+        "block32": lambda x: x.view(-1, 32, 2).transpose(1, 2),
+    }
+    want, stream = None, torch.cuda.Stream()
+    for fmt, encode_as in encoded.items():
+        bufs = [encode_as(x).contiguous() for x in xs]
+        torch.cuda.synchronize()
+        with xg.Correlator(n, f, t, input_format=fmt, channel_offset=off, input_nfrequency=band,
+                           flags=xg.XGPU_DONT_REGISTER) as c:
+            c.tune(1, 0, 0)
+            c.set_stream(stream.cuda_stream)
+            for q in (0, 1, 0):
+                c.run_device(bufs[q].data_ptr())
+            got = c.dump_int64()
+        want = got if want is None else want
+        assert np.array_equal(got, want), fmt

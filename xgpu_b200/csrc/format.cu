@@ -170,7 +170,7 @@ static auto pick_format_host(int state_is_float, bool tiles) {
              : (tiles ? format_host_kernel<false, true> : format_host_kernel<false, false>);
 }
 
-// Conversions are programmatic launches between two engine launches.  Beside the
+// Conversions stand between two engine launches.  Beside the
 // engine launch before it a conversion touches neither that one's input nor its
 // sums, so it starts at once and only ends after it (one block's wait keeps the
 // grid; the others leave their places to the rest); the engine launch behind it
@@ -183,18 +183,23 @@ __device__ __forceinline__ void end_conversion(int beside) {
   if (beside && blockIdx.x == 0) tc::pdl_wait();
 }
 
-// Item u of the compact input (rows of `row` items) in the caller's, whose rows
-// are `pitch` items apart: the band's, of which the context correlates a range.
+// Item u of the compact input (rows of `row` items) in the caller's.  kBand: its rows
+// are `pitch` items apart, the band's, of which the context correlates a range; only
+// then is the division needed before the load can start.  (With it for every input,
+// and 40 registers a thread, six blocks an SM instead of eight, the un-swizzle of
+// N=512, F=64, T=4096 took 194 us alone, and the un-blocking 177; 172 and 168 so.)
+template <bool kBand>
 struct Rows {
   long long row, pitch;
   __device__ __forceinline__ long long at(long long u) const {
-    return row == pitch ? u : u / row * pitch + u % row;
+    return kBand ? u / row * pitch + u % row : u;
   }
 };
 
 // 16 packed samples per thread: one 16-byte load, two 16-byte stores.
-__global__ void unpack4_kernel(const uint4 *in, uint4 *out, long long nquads, Rows rows,
-                               int beside) {
+template <bool kBand>
+__global__ void __launch_bounds__(256, 8)
+    unpack4_kernel(const uint4 *in, uint4 *out, long long nquads, Rows<kBand> rows, int beside) {
   begin_conversion(beside);
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < nquads;
        u += (long long)gridDim.x * blockDim.x) {
@@ -212,15 +217,15 @@ __global__ void unpack4_kernel(const uint4 *in, uint4 *out, long long nquads, Ro
 // takes 16 bytes (input bytes 4e4..4e4+3, four samples each), transposes them
 // 4x4 with byte permutes, and writes one 4-byte word to each of the four
 // sample rows (consecutive threads write consecutive words of a row).
-__global__ void unswizzle_kernel(const uint4 *in, uint32_t *out, long long quads,
-                                 long long row_words, long long pitch, int beside) {
+template <bool kBand>
+__global__ void __launch_bounds__(256, 8)
+    unswizzle_kernel(const uint4 *in, uint32_t *out, long long quads, Rows<kBand> rows, int beside) {
   begin_conversion(beside);
-  // quads = (t/4) * row_words; row_words = f*n (4 bytes per station); pitch: the
-  // same of the band
+  const long long row_words = rows.row;   // f*n, 4 bytes per station; quads = (t/4) * row_words
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < quads;
        u += (long long)gridDim.x * blockDim.x) {
+    const uint4 w = in[rows.at(u)];
     const long long tq = u / row_words, e4 = u - tq * row_words;
-    const uint4 w = in[tq * pitch + e4];
     const uint32_t lo01 = __byte_perm(w.x, w.y, 0x5140), hi01 = __byte_perm(w.x, w.y, 0x7362);
     const uint32_t lo23 = __byte_perm(w.z, w.w, 0x5140), hi23 = __byte_perm(w.z, w.w, 0x7362);
     uint32_t *o = out + 4 * tq * row_words + e4;
@@ -236,8 +241,9 @@ __global__ void unswizzle_kernel(const uint4 *in, uint32_t *out, long long quads
 // shared_transfer_4.cuh:69-86) -> [t][f][s][p]{re,im}.  A 64-byte block holds
 // 16 consecutive (t,f,s) stations: {X.re,Y.re} pairs in bytes 0-31, {X.im,Y.im}
 // pairs in bytes 32-63.  One thread turns 4 stations (8 + 8 bytes) into 16.
-__global__ void unblock32_kernel(const uint2 *in, uint4 *out, long long quads, Rows rows,
-                                 int beside) {
+template <bool kBand>
+__global__ void __launch_bounds__(256, 8)
+    unblock32_kernel(const uint2 *in, uint4 *out, long long quads, Rows<kBand> rows, int beside) {
   begin_conversion(beside);
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < quads;
        u += (long long)gridDim.x * blockDim.x) {
@@ -345,10 +351,15 @@ cudaError_t launch_format(const void *state, int state_is_float, const Sizes &s,
                             (int)s.nbaseline, f0, o);
 }
 
-// A programmatic launch of one of the conversions over `work` thread items.
+// A launch of one of the conversions over `work` thread items, of s's input.
+// Programmatic, except for a long one with nothing to run beside: its blocks would
+// come where the engine launch before it leaves room, and then run as unevenly as
+// they came (un-swizzle and engine of N=512, T=4096 on a caller's stream: F=64 622 us
+// a call, 603 launched plainly, F=16 162 and 159; N=256, F=64, T=1024, 67 MB, 91 either
+// way, F=10 19.7 and 20.7; the other formats gain and lose 1% to 2%).
 template <class... A>
-static cudaError_t launch_conversion(void (*kernel)(A...), long long work, cudaStream_t st,
-                                     A... args) {
+static cudaError_t launch_conversion(void (*kernel)(A..., int), long long work, const Sizes &s,
+                                     bool beside, cudaStream_t st, const A &...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(fmt::grid_for(work, 256));
   cfg.blockDim = dim3(256);
@@ -357,17 +368,23 @@ static cudaError_t launch_conversion(void (*kernel)(A...), long long work, cudaS
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, args...);
+  cfg.numAttrs = beside || 2 * s.vec_length < 128LL << 20 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args..., (int)beside);
 }
 
-cudaError_t load_conversion(int input_format) {
+template <bool kBand>
+static cudaError_t load_conversion_kernel(int input_format) {
   switch (input_format) {
-    case XGPU_INPUT_PACKED4: return load_kernel((const void *)fmt::unpack4_kernel);
-    case XGPU_INPUT_DP4A_SWIZZLED: return load_kernel((const void *)fmt::unswizzle_kernel);
-    case XGPU_INPUT_BLOCK32: return load_kernel((const void *)fmt::unblock32_kernel);
+    case XGPU_INPUT_PACKED4: return load_kernel((const void *)fmt::unpack4_kernel<kBand>);
+    case XGPU_INPUT_DP4A_SWIZZLED: return load_kernel((const void *)fmt::unswizzle_kernel<kBand>);
+    case XGPU_INPUT_BLOCK32: return load_kernel((const void *)fmt::unblock32_kernel<kBand>);
     default: return cudaSuccess;
   }
+}
+
+cudaError_t load_conversion(int input_format, const Sizes &s) {
+  const cudaError_t e = load_conversion_kernel<false>(input_format);
+  return e != cudaSuccess || s.fin == s.f ? e : load_conversion_kernel<true>(input_format);
 }
 
 cudaError_t load_format(int state_is_float, int order) {
@@ -380,25 +397,43 @@ cudaError_t load_format(int state_is_float, int order) {
 cudaError_t launch_unpack4(const uint8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
                            bool beside) {
   // 2n bytes a channel, n a multiple of 16
-  const long long row = (long long)s.f * s.n / 8, quads = row * s.t;
-  return launch_conversion(fmt::unpack4_kernel, quads, st, (const uint4 *)in, (uint4 *)out, quads,
-                           fmt::Rows{row, (long long)s.fin * s.n / 8}, (int)beside);
+  const long long row = (long long)s.f * s.n / 8, pitch = (long long)s.fin * s.n / 8;
+  const long long quads = row * s.t;
+  const uint4 *from = (const uint4 *)in;
+  uint4 *to = (uint4 *)out;
+  if (pitch == row)
+    return launch_conversion<const uint4 *, uint4 *, long long, fmt::Rows<false>>(
+        fmt::unpack4_kernel<false>, quads, s, beside, st, from, to, quads, {row, pitch});
+  return launch_conversion<const uint4 *, uint4 *, long long, fmt::Rows<true>>(
+      fmt::unpack4_kernel<true>, quads, s, beside, st, from, to, quads, {row, pitch});
 }
 
 cudaError_t launch_unswizzle_dp4a(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
                                   bool beside) {
-  const long long row = (long long)s.f * s.n;   // t is a multiple of 4 (ntimepipe % 16 == 0)
+  // t is a multiple of 4 (ntimepipe % 16 == 0)
+  const long long row = (long long)s.f * s.n, pitch = (long long)s.fin * s.n;
   const long long quads = (long long)(s.t / 4) * row;
-  return launch_conversion(fmt::unswizzle_kernel, quads, st, (const uint4 *)in, (uint32_t *)out,
-                           quads, row, (long long)s.fin * s.n, (int)beside);
+  const uint4 *from = (const uint4 *)in;
+  uint32_t *to = (uint32_t *)out;
+  if (pitch == row)
+    return launch_conversion<const uint4 *, uint32_t *, long long, fmt::Rows<false>>(
+        fmt::unswizzle_kernel<false>, quads, s, beside, st, from, to, quads, {row, pitch});
+  return launch_conversion<const uint4 *, uint32_t *, long long, fmt::Rows<true>>(
+      fmt::unswizzle_kernel<true>, quads, s, beside, st, from, to, quads, {row, pitch});
 }
 
 cudaError_t launch_unblock32(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
                              bool beside) {
-  const long long row = (long long)s.f * s.n / 16;   // blocks of 16 stations
+  // blocks of 16 stations
+  const long long row = (long long)s.f * s.n / 16, pitch = (long long)s.fin * s.n / 16;
   const long long quads = 4 * row * s.t;
-  return launch_conversion(fmt::unblock32_kernel, quads, st, (const uint2 *)in, (uint4 *)out, quads,
-                           fmt::Rows{row, (long long)s.fin * s.n / 16}, (int)beside);
+  const uint2 *from = (const uint2 *)in;
+  uint4 *to = (uint4 *)out;
+  if (pitch == row)
+    return launch_conversion<const uint2 *, uint4 *, long long, fmt::Rows<false>>(
+        fmt::unblock32_kernel<false>, quads, s, beside, st, from, to, quads, {row, pitch});
+  return launch_conversion<const uint2 *, uint4 *, long long, fmt::Rows<true>>(
+      fmt::unblock32_kernel<true>, quads, s, beside, st, from, to, quads, {row, pitch});
 }
 
 void gauss_thresholds(double sigma, uint32_t thr[254]) {

@@ -206,9 +206,9 @@ cudaError_t launch_unblock32(const int8_t *in, int8_t *out, const Sizes &s, cuda
 // host memory.
 cudaError_t launch_format(const void *state, int state_is_float, const Sizes &s, const DumpOut &o,
                           cudaStream_t st, int f0 = 0, int fcount = -1, bool host_out = false);
-// Load the kernels that the conversions and launch_format launch for a context's input format, and for
-// its buffer's type and its matrix order.
-cudaError_t load_conversion(int input_format);
+// Load the kernels that the conversions launch for a context's input format, and
+// launch_format for its buffer's type and its matrix order.
+cudaError_t load_conversion(int input_format, const Sizes &s);
 cudaError_t load_format(int state_is_float, int order);
 cudaError_t launch_generate(void *out, size_t nbytes, int kind, unsigned long long seed,
                             double sigma, cudaStream_t st);

@@ -836,7 +836,7 @@ int xgpuInitEx(XGPUContext *context, int device_flags, const XGPUConfig *cfg_in)
     return fail(XGPU_CUDA_ERROR);
   }
   if ((cfg.engine == XGPU_ENGINE_PLAIN && plain_configure_device() != cudaSuccess) ||
-      load_conversion((int)cfg.input_format) != cudaSuccess ||
+      load_conversion((int)cfg.input_format, in->sz) != cudaSuccess ||
       load_format(in->int_state ? 0 : 1, (int)cfg.matrix_order) != cudaSuccess) {
     cudaGetLastError();
     return fail(XGPU_CUDA_ERROR);
