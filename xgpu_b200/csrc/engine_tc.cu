@@ -518,7 +518,6 @@ cudaError_t tc_check_device() {
 
 int tc_fill_job(Job *job, const void *dev_in, const Sizes &s, int t0, int tcount, int64_t *state,
                 int store, int ksplit, int item_begin, int pair) {
-  if (make_tc_tensor_map(&job->map, dev_in, s) != 0) return -1;
   const long long tile = pair ? 2 * tc::kTile : tc::kTile;
   const long long ntl = (4LL * s.n + tile - 1) / tile;
   const long long npairs = ntl * (ntl + 1) / 2;
@@ -526,7 +525,9 @@ int tc_fill_job(Job *job, const void *dev_in, const Sizes &s, int t0, int tcount
   if (ksplit < 1) ksplit = 1;
   if (ksplit > total_steps) ksplit = total_steps;
   const int per = (total_steps + ksplit - 1) / ksplit;
+  if (per > kMaxItemSteps) return kItemTooLong;
   ksplit = (total_steps + per - 1) / per;   // every split non-empty
+  if (make_tc_tensor_map(&job->map, dev_in, s) != 0) return -1;
   if ((long long)s.f * npairs * ksplit + item_begin > 0x7fffffffLL) return -2;
   job->state = state;
   job->nbaseline = s.nbaseline;
@@ -560,6 +561,11 @@ cudaError_t launch_tc_tuned(const CUtensorMap &map, const Sizes &s, int t0, int 
     return launch_tc2(map, s, t0, tcount, state, overwrite, err, st, tune, overlap, f0, fcount,
                       packed_in, words, words_store);
   if (packed_in) return cudaErrorInvalidValue;   // only the CTA-pair kernel expands packed input
+  const int total_steps = (tcount + tc::kKt - 1) / tc::kKt;
+  int ksplit = tune.ksplit < 1 ? 1 : (tune.ksplit > total_steps ? total_steps : tune.ksplit);
+  const int per = (total_steps + ksplit - 1) / ksplit;
+  if (per > kMaxItemSteps) return cudaErrorInvalidValue;
+  ksplit = (total_steps + per - 1) / per;
   const int sms = current_device_sms();
   if (!sms) return cudaErrorInvalidDevice;
   {
@@ -572,10 +578,6 @@ cudaError_t launch_tc_tuned(const CUtensorMap &map, const Sizes &s, int t0, int 
   Job &j = p.single;
   const long long ntl = (4LL * s.n + tc::kTile - 1) / tc::kTile;
   const long long npairs = ntl * (ntl + 1) / 2;
-  const int total_steps = (tcount + tc::kKt - 1) / tc::kKt;
-  int ksplit = tune.ksplit < 1 ? 1 : (tune.ksplit > total_steps ? total_steps : tune.ksplit);
-  const int per = (total_steps + ksplit - 1) / ksplit;
-  ksplit = (total_steps + per - 1) / per;
   if ((long long)fcount * npairs * ksplit > 0x7fffffffLL) return cudaErrorInvalidValue;
   // Split items of one tile all add into the buffer: a zero buffer must be
   // cleared first (its channel range) when it would otherwise be stored into.

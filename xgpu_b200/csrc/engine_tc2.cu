@@ -1008,6 +1008,11 @@ cudaError_t launch_tc2(const CUtensorMap &map, const Sizes &s, int t0, int tcoun
   if (fcount < 0) fcount = s.f - f0;
   if (f0 < 0 || fcount < 1 || f0 + fcount > s.f) return cudaErrorInvalidValue;
   const bool packed = packed_in != nullptr;   // `map` describes it (make_packed_map)
+  const int total_steps = (tcount + tc2::kKt - 1) / tc2::kKt;
+  int ksplit = tune.ksplit < 1 ? 1 : (tune.ksplit > total_steps ? total_steps : tune.ksplit);
+  const int per = (total_steps + ksplit - 1) / ksplit;
+  if (per > kMaxItemSteps) return cudaErrorInvalidValue;
+  ksplit = (total_steps + per - 1) / per;
   const int num_sms = current_device_sms();
   if (!num_sms) return cudaErrorInvalidDevice;
   {
@@ -1019,10 +1024,6 @@ cudaError_t launch_tc2(const CUtensorMap &map, const Sizes &s, int t0, int tcoun
   j.map = map;
   const long long ntl = (4LL * s.n + 2 * tc2::kHalf - 1) / (2 * tc2::kHalf);
   const long long npairs = ntl * (ntl + 1) / 2;
-  const int total_steps = (tcount + tc2::kKt - 1) / tc2::kKt;
-  int ksplit = tune.ksplit < 1 ? 1 : (tune.ksplit > total_steps ? total_steps : tune.ksplit);
-  const int per = (total_steps + ksplit - 1) / ksplit;
-  ksplit = (total_steps + per - 1) / per;
   if ((long long)fcount * npairs * ksplit > 0x7fffffffLL) return cudaErrorInvalidValue;
   if (overwrite && ksplit > 1) {
     const size_t per_channel = (size_t)s.state_elems / s.f;   // int64 words

@@ -18,6 +18,10 @@ constexpr int kNpol = 2;
 // a real or imaginary part at full scale -128), so the int32 accumulators stay
 // exact; each launch adds into the int64 integration buffer.
 constexpr int kSegment = 32768;
+// The most stages of a tensor-core work item: its drain forms re and im in 32 bits.
+// What fills a job or launches one refuses longer items.
+constexpr int kMaxItemSteps = kSegment / kTcSamplesPerStage;
+constexpr int kItemTooLong = -3;   // of tc_fill_job
 
 // Device error codes written by kernels into the context's error word.
 enum DeviceError : int {

@@ -190,7 +190,7 @@ __device__ __forceinline__ void pdl_wait() {
 // lane makes product p2 = 0, the imaginary-row lane (its neighbour) p2 = 1; each
 // needs two values of the other:
 //   re = G(re, re) + G(im, im), im = G(im, re) - G(re, im).
-// In 32 bits: the accumulators hold at most kSegment samples, so that re and im
+// In 32 bits: an item has at most kSegment samples (kMaxItemSteps), so that re and im
 // stay within 2^30; a third of the instructions of the 64-bit form.  A drain of
 // 128 columns, which four warps with nothing to hide behind spend on the
 // dependent instructions of this, took 1.65 us with that and takes 1.15.
