@@ -545,12 +545,6 @@ int tc_fill_job(Job *job, const void *dev_in, const Sizes &s, int t0, int tcount
   return 0;
 }
 
-cudaError_t launch_tc(const CUtensorMap &map, const Sizes &s, int t0, int tcount, int64_t *state,
-                      int overwrite, int *err, cudaStream_t st) {
-  TcTuning tune;   // single CTAs, no time split, one CTA per SM
-  return launch_tc_tuned(map, s, t0, tcount, state, overwrite, err, st, tune, 0);
-}
-
 cudaError_t launch_tc_tuned(const CUtensorMap &map, const Sizes &s, int t0, int tcount,
                             int64_t *state, int overwrite, int *err, cudaStream_t st,
                             const TcTuning &tune, int overlap, int f0, int fcount,

@@ -616,7 +616,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPacked ? kThreadsPa
 #pragma unroll
             for (int jj = 0; jj < 8; ++jj) {
               const int2 x = unscale<kPacked>(combine((int)v[q][4 * jj], (int)v[q][4 * jj + 1],
-                                                             (int)v[q][4 * jj + 2], (int)v[q][4 * jj + 3], c));
+                                                      (int)v[q][4 * jj + 2], (int)v[q][4 * jj + 3], c));
               const int jl = q * 8 + jj;
               if (jl < jmax) *(int4 *)(srow + jl * 64) = make_int4(x.x, x.x >> 31, x.y, x.y >> 31);
             }
@@ -745,7 +745,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPacked ? kThreadsPa
 #pragma unroll
             for (int jj = 0; jj < 8; ++jj) {
               const int2 x = unscale<kPacked>(combine((int)v[q][4 * jj], (int)v[q][4 * jj + 1],
-                                                             (int)v[q][4 * jj + 2], (int)v[q][4 * jj + 3], c));
+                                                      (int)v[q][4 * jj + 2], (int)v[q][4 * jj + 3], c));
               const int jl = q * 8 + jj;
               if (jl < jmax) *(int4 *)(srow + jl * 64) = make_int4(x.x, x.x >> 31, x.y, x.y >> 31);
             }

@@ -87,8 +87,6 @@ cudaError_t launch_plain_fp32(const int8_t *in, const Sizes &s, int t0, int tcou
                               int stall = 0, int f0 = 0, int fcount = -1);
 
 // Tensor-core engine.  The tensor map describes `in` (see make_tc_tensor_map).
-cudaError_t launch_tc(const CUtensorMap &map, const Sizes &s, int t0, int tcount,
-                      int64_t *state, int overwrite, int *err, cudaStream_t st);
 // Launched programmatically (PDL): the prologue overlaps the previous kernel of
 // the stream.  overlap = 1 promises that the previous kernel of the stream is
 // an engine launch of the same integration that does not store (only adds)
@@ -115,7 +113,7 @@ cudaError_t launch_tc2(const CUtensorMap &map, const Sizes &s, int t0, int tcoun
                        int overwrite, int *err, cudaStream_t st, const TcTuning &tune,
                        int overlap, int f0 = 0, int fcount = -1,
                        const void *packed_in = nullptr, uint64_t *words = nullptr,
-                            int words_store = 0);
+                       int words_store = 0);
 // Word buffer: 64-bit words (im * 2^32 + re of one visibility's sums) in
 // 32 x 32-station blocks; its size for sizes s, and the fold that adds the
 // words into the int64 buffer (triangular order).  Exact while every sum in
