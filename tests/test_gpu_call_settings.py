@@ -125,4 +125,4 @@ def test_lone_packed_calls_expand_in_the_kernel(launches, how):
 
 def test_chained_packed_calls_convert_ahead(launches):
     names = [name for name, grid in launches["packed chain"]]
-    assert names[-6:] == 3 * ["unpack4_kernel", "xengine_tc2_kernel<false, false>"]
+    assert names[-6:] == 3 * ["unpack4_kernel<false>", "xengine_tc2_kernel<false, false>"]
