@@ -75,6 +75,9 @@ calls(c, x, 3)
 torch.cuda.synchronize()
 out["packed chain"] = recorded(lambda: calls(c, x, 4))
 c.close()
+c, x = context(384, 64, 8192, "packed4")    # 86,016 stages of six tile rows
+out["packed chain, six rows"] = recorded(lambda: calls(c, x, 4))
+c.close()
 for name, sync in (("first", xg.SYNCOP_NONE), ("first transfer", xg.SYNCOP_SYNC_TRANSFER),
                    ("first waited", xg.SYNCOP_SYNC_COMPUTE)):
     c, x = context(400, 5, 384)    # short items: a call that may be one of many uses the words
@@ -126,3 +129,8 @@ def test_lone_packed_calls_expand_in_the_kernel(launches, how):
 def test_chained_packed_calls_convert_ahead(launches):
     names = [name for name, grid in launches["packed chain"]]
     assert names[-6:] == 3 * ["unpack4_kernel<false>", "xengine_tc2_kernel<false, false>"]
+
+
+def test_chained_packed_calls_of_few_tile_rows_expand_in_the_kernel(launches):
+    names = [name for name, grid in launches["packed chain, six rows"]]
+    assert names == 4 * ["xengine_tc2_kernel<true, false>"]

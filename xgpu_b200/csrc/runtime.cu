@@ -322,19 +322,22 @@ TcTuning call_tuning(Internal *in, bool waited) {
 // caller's stream it could not.  Shorter calls overlap one another, which converted
 // ones do not (N=256, F=32, T=4096, 10,240 stages: 16 calls 1.43 against 1.61 ms).
 // Chains with their dump, N=512, T=8192, F=64 (147,456 stages): 8 calls 14.7 to 13.2
-// ms; F=16 (36,864): 4 and 8 calls 2.59 to 2.46 and 3.79 to 3.44; N=768, F=16
-// (79,872) 8.17 to 7.34, N=384, F=24, T=6144 (24,192) no gain.  Under the power cap,
-// after seconds without a pause, it draws the clock down and gives less: chains of
-// 16 at N=512, F=64 1.21 to 1.19 ms a call, F=16 306 to 296 us, of 4 at F=64 1.21 to
-// 1.23, F=256 4.87 to 4.91.  A call by itself only has it to pay for then (N=512,
-// F=64 1.25 to 1.34 ms, F=24 486 to 509 us), so calls that find nothing before
-// them, or came one by one last time, expand in the kernel.
+// ms; F=16 (36,864): 4 and 8 calls 2.59 to 2.46 and 3.79 to 3.44 ms.
+// That is in bursts.  After seconds without a pause the power cap sets the clock, and
+// the conversion's traffic costs some of it: 6 bytes a station and sample, against the
+// stages of a triangle of 256 x 256 tiles.  Time of chains with it over that without,
+// in bursts and under the cap (by box), T=8192: N=640, F=40 0.81 and 0.93, N=576, F=48
+// 0.82 and 0.94, N=512, F=48 0.85 and 0.97, F=96 0.86 and 0.97-1.03, F=256 0.89 and
+// 0.99-1.05, N=448, F=80 0.86 and 0.99, N=384, F=96 0.97 and 1.09, N=256, F=96 1.10 and
+// 1.21: not below seven tile rows.  A call by itself only has it to pay for (N=512,
+// F=64 1.25 to 1.34 ms under the cap, F=24 486 to 509 us), so calls that find nothing
+// before them, or came one by one last time, expand in the kernel.
 bool unpack_ahead(Internal *in) {
   if (in->cfg.input_format != XGPU_INPUT_PACKED4 || !in->int_state || !in->use.wide ||
       in->s_comp != in->s_own)
     return false;
   const long long stages = tc2_stages(in->szc);
-  if (stages < 30000) return false;
+  if (stages < 30000 || in->szc.n <= 6 * 64) return false;
   if (in->chain > 0 && own_stream_idle(in)) end_chain(in);
   return stages >= 100000 ? in->chain > 0 || in->chain_before > 1 : in->chain >= 2;
 }
