@@ -19,7 +19,7 @@ import torch
 from torch.profiler import profile, ProfilerActivity
 import xgpu_b200 as xg
 
-def recorded(f):
+def recorded(f, times=0):
     with profile(activities=[ProfilerActivity.CUDA]) as p:
         f()
         torch.cuda.synchronize()
@@ -28,10 +28,11 @@ def recorded(f):
     with open(path) as fh:
         ev = [e for e in json.load(fh)["traceEvents"] if e.get("cat") == "kernel"]
     ev.sort(key=lambda e: e["ts"])
-    return [[e["name"].split("(")[0].split("::")[-1], e["args"]["grid"][0]] for e in ev]
+    return [[e["name"].split("(")[0].split("::")[-1], e["args"]["grid"][0]] + times * [e["ts"], e["ts"] + e["dur"]]
+            for e in ev]
 
-def context(n, f, t, fmt="int8"):
-    c = xg.Correlator(n, f, t, input_format=fmt, flags=xg.XGPU_DONT_REGISTER)
+def context(n, f, t, fmt="int8", **kind):
+    c = xg.Correlator(n, f, t, input_format=fmt, **kind, flags=xg.XGPU_DONT_REGISTER)
     x = torch.randint(-8, 8, (4 * n * f * t,), device="cuda", dtype=torch.int8)
     torch.cuda.synchronize()
     return c, x
@@ -78,6 +79,12 @@ c.close()
 c, x = context(384, 64, 8192, "packed4")    # 86,016 stages of six tile rows
 out["packed chain, six rows"] = recorded(lambda: calls(c, x, 4))
 c.close()
+for name, kind in (("dp4a", {}), ("fp32", {"compute": "fp32", "output": "float32"})):
+    c, x = context(64, 10, 1024, "dp4a_swizzled", engine="plain", **kind)
+    calls(c, x, 4)
+    torch.cuda.synchronize()
+    out["converted " + name] = recorded(lambda: calls(c, x, 8), times=1)
+    c.close()
 for name, sync in (("first", xg.SYNCOP_NONE), ("first transfer", xg.SYNCOP_SYNC_TRANSFER),
                    ("first waited", xg.SYNCOP_SYNC_COMPUTE)):
     c, x = context(400, 5, 384)    # short items: a call that may be one of many uses the words
@@ -134,3 +141,16 @@ def test_chained_packed_calls_convert_ahead(launches):
 def test_chained_packed_calls_of_few_tile_rows_expand_in_the_kernel(launches):
     names = [name for name, grid in launches["packed chain, six rows"]]
     assert names == 4 * ["xengine_tc2_kernel<true, false>"]
+
+
+@pytest.mark.parametrize("engine", ["dp4a", "fp32"])
+def test_small_plain_grids_come_after_their_conversion(launches, engine):
+    """Let in beside the conversion, their CTAs would crowd on the SMs that it leaves
+    room on."""
+    rows = launches["converted " + engine]
+    assert len(rows) == 16
+    for conversion, launch in zip(rows[::2], rows[1::2]):
+        assert "unswizzle" in conversion[0] and engine in launch[0]
+        # times in us: a few for the launch itself, where the conversion that waits for
+        # the launch before takes 15 to 30
+        assert launch[2] > conversion[3] - 4

@@ -59,6 +59,20 @@ def test_host_and_device_calls_in_turn(xg, oracle_mod, fmt, engine, sync):
         assert np.array_equal(c.dump_int64(), want)
 
 
+@pytest.mark.parametrize("compute", ["int8", "fp32"])
+@pytest.mark.parametrize("fmt", ["packed4", "dp4a_swizzled", "block32"])
+def test_plain_grids_that_fill_the_gpu(xg, oracle_mod, fmt, compute):
+    """648 blocks: their launches come at the conversion's start."""
+    n, f, t = 256, 9, 128
+    host, dev, sums = inputs(oracle_mod, fmt, n, f, t, 4, 500)
+    out = "int32" if compute == "int8" else "float32"
+    with xg.Correlator(n, f, t, ntimepipe=16, engine="plain", compute=compute, output=out,
+                       input_format=fmt) as c:
+        for q in range(8):
+            c.run_device(dev[q % 4].data_ptr())
+        assert np.array_equal(c.dump(), (2 * sum(sums)).astype(out))
+
+
 @pytest.mark.parametrize("band,off", [(0, 0), (18, 1)])
 def test_long_calls_on_a_callers_stream(xg, band, off):
     """134 MB of int8 samples a call, converted with nothing beside: launched plainly.

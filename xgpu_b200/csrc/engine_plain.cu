@@ -818,6 +818,11 @@ static dim3 plain_grid(const Sizes &s, int fcount, int ksplit = 1) {
   return dim3((unsigned)blocks, (unsigned)fcount, (unsigned)ksplit);
 }
 
+long long plain_blocks(const Sizes &s) {
+  const dim3 g = plain_grid(s, s.f);
+  return (long long)g.x * g.y;
+}
+
 // Time splits of a dp4a launch: enough CTAs for one wave of resident CTAs
 // (five per SM), or for half of one when the launch may overlap the previous
 // adding launch (whose last CTAs, and the next launch's, fill the rest; each

@@ -170,17 +170,23 @@ static auto pick_format_host(int state_is_float, bool tiles) {
              : (tiles ? format_host_kernel<false, true> : format_host_kernel<false, false>);
 }
 
-// Conversions stand between two engine launches.  Beside the
-// engine launch before it a conversion touches neither that one's input nor its
-// sums, so it starts at once and only ends after it (one block's wait keeps the
-// grid; the others leave their places to the rest); the engine launch behind it
-// waits for the conversion, and so for both.
-__device__ __forceinline__ void begin_conversion(int beside) {
-  if (!beside) tc::pdl_wait();
-  tc::pdl_trigger();
+// Conversions stand between two engine launches.  Beside the engine launch before it
+// a conversion touches neither that one's input nor its sums, so it starts at once
+// and only ends after it (one block's wait keeps the grid; the others leave their
+// places to the rest); the engine launch behind it waits for the conversion, and so
+// for both.  That launch comes early, its prologue under the conversion, where its CTAs
+// can only spread evenly: one fills an SM, or they fill all places.  CTAs of smaller
+// grids, several of which fit an SM, would settle where the conversion's blocks leave
+// room and then run as unevenly (kConvertLate: they come when it is done).  Plain
+// engines, us a call in chains early and late: dp4a, swizzled, N=64, F=10, T=1024 30.2
+// and 17.9, N=96, F=16, T=512 31.1 and 22.7, N=256, F=10 (720 CTAs) 106.1 and 107.2;
+// FP32, packed, N=128, F=10 50.9 and 40.9, N=176, F=13, T=1552 172 and 143.
+__device__ __forceinline__ void begin_conversion(int mode) {
+  if (!(mode & kConvertBeside)) tc::pdl_wait();
+  if (!(mode & kConvertLate)) tc::pdl_trigger();
 }
-__device__ __forceinline__ void end_conversion(int beside) {
-  if (beside && blockIdx.x == 0) tc::pdl_wait();
+__device__ __forceinline__ void end_conversion(int mode) {
+  if ((mode & kConvertBeside) && blockIdx.x == 0) tc::pdl_wait();
 }
 
 // Item u of the compact input (rows of `row` items) in the caller's.  kBand: its rows
@@ -199,8 +205,8 @@ struct Rows {
 // 16 packed samples per thread: one 16-byte load, two 16-byte stores.
 template <bool kBand>
 __global__ void __launch_bounds__(256, 8)
-    unpack4_kernel(const uint4 *in, uint4 *out, long long nquads, Rows<kBand> rows, int beside) {
-  begin_conversion(beside);
+    unpack4_kernel(const uint4 *in, uint4 *out, long long nquads, Rows<kBand> rows, int mode) {
+  begin_conversion(mode);
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < nquads;
        u += (long long)gridDim.x * blockDim.x) {
     const uint4 w = in[rows.at(u)];
@@ -209,7 +215,7 @@ __global__ void __launch_bounds__(256, 8)
     out[2 * u] = make_uint4(a.x, a.y, b.x, b.y);
     out[2 * u + 1] = make_uint4(c.x, c.y, d.x, d.y);
   }
-  end_conversion(beside);
+  end_conversion(mode);
 }
 
 // xgpuSwizzleInput's layout (cpu_util.c:235-255) back to [t][f][s][p][c]:
@@ -219,8 +225,8 @@ __global__ void __launch_bounds__(256, 8)
 // sample rows (consecutive threads write consecutive words of a row).
 template <bool kBand>
 __global__ void __launch_bounds__(256, 8)
-    unswizzle_kernel(const uint4 *in, uint32_t *out, long long quads, Rows<kBand> rows, int beside) {
-  begin_conversion(beside);
+    unswizzle_kernel(const uint4 *in, uint32_t *out, long long quads, Rows<kBand> rows, int mode) {
+  begin_conversion(mode);
   const long long row_words = rows.row;   // f*n, 4 bytes per station; quads = (t/4) * row_words
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < quads;
        u += (long long)gridDim.x * blockDim.x) {
@@ -234,7 +240,7 @@ __global__ void __launch_bounds__(256, 8)
     o[2 * row_words] = __byte_perm(hi01, hi23, 0x5410);
     o[3 * row_words] = __byte_perm(hi01, hi23, 0x7632);
   }
-  end_conversion(beside);
+  end_conversion(mode);
 }
 
 // xGPU's COMPLEX_BLOCK_SIZE=32 input (read by omp_xengine.c:61-78,
@@ -243,8 +249,8 @@ __global__ void __launch_bounds__(256, 8)
 // pairs in bytes 32-63.  One thread turns 4 stations (8 + 8 bytes) into 16.
 template <bool kBand>
 __global__ void __launch_bounds__(256, 8)
-    unblock32_kernel(const uint2 *in, uint4 *out, long long quads, Rows<kBand> rows, int beside) {
-  begin_conversion(beside);
+    unblock32_kernel(const uint2 *in, uint4 *out, long long quads, Rows<kBand> rows, int mode) {
+  begin_conversion(mode);
   for (long long u = blockIdx.x * (long long)blockDim.x + threadIdx.x; u < quads;
        u += (long long)gridDim.x * blockDim.x) {
     const long long blk = rows.at(u >> 2);   // rows of whole blocks (n is a multiple of 16)
@@ -258,7 +264,7 @@ __global__ void __launch_bounds__(256, 8)
     o.w = __byte_perm(re.y, im.y, 0x7362);
     out[u] = o;
   }
-  end_conversion(beside);
+  end_conversion(mode);
 }
 
 // Seeded synthetic bytes; the same hash and tables as the host generator.
@@ -359,7 +365,7 @@ cudaError_t launch_format(const void *state, int state_is_float, const Sizes &s,
 // way, F=10 19.7 and 20.7; the other formats gain and lose 1% to 2%).
 template <class... A>
 static cudaError_t launch_conversion(void (*kernel)(A..., int), long long work, const Sizes &s,
-                                     bool beside, cudaStream_t st, const A &...args) {
+                                     int mode, cudaStream_t st, const A &...args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(fmt::grid_for(work, 256));
   cfg.blockDim = dim3(256);
@@ -368,8 +374,8 @@ static cudaError_t launch_conversion(void (*kernel)(A..., int), long long work, 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = beside || 2 * s.vec_length < 128LL << 20 ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, args..., (int)beside);
+  cfg.numAttrs = (mode & kConvertBeside) || 2 * s.vec_length < 128LL << 20 ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args..., mode);
 }
 
 template <bool kBand>
@@ -395,7 +401,7 @@ cudaError_t load_format(int state_is_float, int order) {
 }
 
 cudaError_t launch_unpack4(const uint8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
-                           bool beside) {
+                           int mode) {
   // 2n bytes a channel, n a multiple of 16
   const long long row = (long long)s.f * s.n / 8, pitch = (long long)s.fin * s.n / 8;
   const long long quads = row * s.t;
@@ -403,13 +409,13 @@ cudaError_t launch_unpack4(const uint8_t *in, int8_t *out, const Sizes &s, cudaS
   uint4 *to = (uint4 *)out;
   if (pitch == row)
     return launch_conversion<const uint4 *, uint4 *, long long, fmt::Rows<false>>(
-        fmt::unpack4_kernel<false>, quads, s, beside, st, from, to, quads, {row, pitch});
+        fmt::unpack4_kernel<false>, quads, s, mode, st, from, to, quads, {row, pitch});
   return launch_conversion<const uint4 *, uint4 *, long long, fmt::Rows<true>>(
-      fmt::unpack4_kernel<true>, quads, s, beside, st, from, to, quads, {row, pitch});
+      fmt::unpack4_kernel<true>, quads, s, mode, st, from, to, quads, {row, pitch});
 }
 
 cudaError_t launch_unswizzle_dp4a(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
-                                  bool beside) {
+                                  int mode) {
   // t is a multiple of 4 (ntimepipe % 16 == 0)
   const long long row = (long long)s.f * s.n, pitch = (long long)s.fin * s.n;
   const long long quads = (long long)(s.t / 4) * row;
@@ -417,13 +423,13 @@ cudaError_t launch_unswizzle_dp4a(const int8_t *in, int8_t *out, const Sizes &s,
   uint32_t *to = (uint32_t *)out;
   if (pitch == row)
     return launch_conversion<const uint4 *, uint32_t *, long long, fmt::Rows<false>>(
-        fmt::unswizzle_kernel<false>, quads, s, beside, st, from, to, quads, {row, pitch});
+        fmt::unswizzle_kernel<false>, quads, s, mode, st, from, to, quads, {row, pitch});
   return launch_conversion<const uint4 *, uint32_t *, long long, fmt::Rows<true>>(
-      fmt::unswizzle_kernel<true>, quads, s, beside, st, from, to, quads, {row, pitch});
+      fmt::unswizzle_kernel<true>, quads, s, mode, st, from, to, quads, {row, pitch});
 }
 
 cudaError_t launch_unblock32(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
-                             bool beside) {
+                             int mode) {
   // blocks of 16 stations
   const long long row = (long long)s.f * s.n / 16, pitch = (long long)s.fin * s.n / 16;
   const long long quads = 4 * row * s.t;
@@ -431,9 +437,9 @@ cudaError_t launch_unblock32(const int8_t *in, int8_t *out, const Sizes &s, cuda
   uint4 *to = (uint4 *)out;
   if (pitch == row)
     return launch_conversion<const uint2 *, uint4 *, long long, fmt::Rows<false>>(
-        fmt::unblock32_kernel<false>, quads, s, beside, st, from, to, quads, {row, pitch});
+        fmt::unblock32_kernel<false>, quads, s, mode, st, from, to, quads, {row, pitch});
   return launch_conversion<const uint2 *, uint4 *, long long, fmt::Rows<true>>(
-      fmt::unblock32_kernel<true>, quads, s, beside, st, from, to, quads, {row, pitch});
+      fmt::unblock32_kernel<true>, quads, s, mode, st, from, to, quads, {row, pitch});
 }
 
 void gauss_thresholds(double sigma, uint32_t thr[254]) {

@@ -190,18 +190,22 @@ int current_device_sms();
 cudaError_t tc_configure_device();
 cudaError_t tc2_set_smem_attribute();
 cudaError_t plain_configure_device();
+// CTAs of a plain engine's launch over all of s, without time splits.
+long long plain_blocks(const Sizes &s);
 
 // ---- input conversion, output formatting, synthetic input -----------------
 // `in` holds s.fin channels per row and points at the first that the context
-// correlates; `out` is compact.  Launched programmatically.  beside: the launch
+// correlates; `out` is compact.  mode: kConvertBeside, the launch
 // before it on `st` is an engine launch that reads neither `in` (complete
 // already) nor `out`: the conversion runs beside it, and waits for it at its end.
+// kConvertLate, the launch behind it comes when the conversion is done, not at its start.
+constexpr int kConvertBeside = 1, kConvertLate = 2;
 cudaError_t launch_unpack4(const uint8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
-                           bool beside);
+                           int mode);
 cudaError_t launch_unswizzle_dp4a(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
-                                  bool beside);
+                                  int mode);
 cudaError_t launch_unblock32(const int8_t *in, int8_t *out, const Sizes &s, cudaStream_t st,
-                             bool beside);
+                             int mode);
 // Channels [f0, f0 + fcount) of the buffer (int64 or float) into o.out in its
 // order and type (fcount < 0: through the last channel; other channels' words
 // are untouched).  Launched programmatically.  host_out: the output is mapped

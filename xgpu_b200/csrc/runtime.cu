@@ -475,15 +475,17 @@ int run_engine(Internal *in, const void *d_input, cudaEvent_t input_ready, bool 
     if (input_ready) XGPU_CHECK(cudaStreamWaitEvent(in->s_comp, input_ready, 0));
     // On the context's own stream the caller's input is complete already; on a
     // caller's stream the work before the call may still be making it.
-    const bool beside = engine_tail && !input_ready;
+    int mode = engine_tail && !input_ready ? kConvertBeside : 0;
+    if (in->cfg.engine == XGPU_ENGINE_PLAIN && plain_blocks(in->szc) < 4LL * current_device_sms())
+      mode |= kConvertLate;
     const Sizes &from = ranged ? s : in->szc;
     const int8_t *src = x + (ranged ? s.fin0 * s.chan_bytes : 0);
     if (in->cfg.input_format == XGPU_INPUT_PACKED4)
-      XGPU_CHECK(launch_unpack4((const uint8_t *)src, in->d_conv[conv], from, in->s_comp, beside));
+      XGPU_CHECK(launch_unpack4((const uint8_t *)src, in->d_conv[conv], from, in->s_comp, mode));
     else if (in->cfg.input_format == XGPU_INPUT_BLOCK32)
-      XGPU_CHECK(launch_unblock32(src, in->d_conv[conv], from, in->s_comp, beside));
+      XGPU_CHECK(launch_unblock32(src, in->d_conv[conv], from, in->s_comp, mode));
     else
-      XGPU_CHECK(launch_unswizzle_dp4a(src, in->d_conv[conv], from, in->s_comp, beside));
+      XGPU_CHECK(launch_unswizzle_dp4a(src, in->d_conv[conv], from, in->s_comp, mode));
     x = in->d_conv[conv];
   } else {
     if (input_ready) XGPU_CHECK(cudaStreamWaitEvent(in->s_comp, input_ready, 0));
