@@ -494,8 +494,8 @@ def bench_large_array(xg, torch, device, blocks=64, check_channels=(0, F3 - 1)):
     import oracle
     out = {"nstation": N3, "nfrequency": F3, "ntime": T3, "blocks": blocks}
     for fmt, kind, sig in (("packed4", 1, 0.0), ("int8", 0, 40.0)):
-        # The context's own streams (packed input is expanded on a side stream
-        # before each block's correlation); timed by the host around a
+        # The context's own streams (packed input is expanded ahead of each block's
+        # launch, beside the block before); timed by the host around a
         # synchronised 64-block run (hundreds of ms).
         c = xg.Correlator(N3, F3, T3, ntimepipe=128, engine="tensor", input_format=fmt,
                           device=device)

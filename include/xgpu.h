@@ -348,14 +348,18 @@ int xgpuCorrelateStatic(const void *device_input, void *device_output, const XGP
  * in chains of calls that overlap as a stream of calls does and read their
  * input from device memory rather than the L2 cache (temporary buffers of up
  * to about 256 MB plus one integration buffer, freed before it returns), and
- * the fastest setting is kept.  With CTA pairs, XGPU_INPUT_PACKED4 input
- * is expanded inside the kernel, except for long calls, whose input a pre-pass
- * converts beside the previous call; the other kernels read an int8 copy that a
- * pre-pass makes. */
+ * the fastest setting is kept.  A context that was never tuned chooses per call:
+ * its default (CTA pairs from 384 stations on, single CTAs below, every SM), or CTA
+ * pairs on part of the SMs for calls that overlap those before them; any xgpuTune
+ * fixes one setting for every call.  With CTA pairs, XGPU_INPUT_PACKED4 input
+ * is expanded inside the kernel, except in chains of long calls of more than 384
+ * stations, whose input a pre-pass converts beside the previous call; the other
+ * kernels read an int8 copy that a pre-pass makes. */
 int xgpuTune(XGPUContext *context, int ksplit, int grid, int pair);
 
-/* The setting in use (as xgpuTune takes it; ksplit >= 1), e.g. to keep an
- * autotuned choice and pass it to xgpuTune in a later run. */
+/* The setting that xgpuTune chose (as xgpuTune takes it; ksplit >= 1), e.g. to keep
+ * an autotuned choice and pass it to xgpuTune in a later run.  For a context that
+ * was never tuned, the default that it starts from, not what each call chose. */
 int xgpuTuning(XGPUContext *context, int *ksplit, int *grid, int *pair);
 
 /* Test hook, for testing a caller's error handling.  While enabled, the

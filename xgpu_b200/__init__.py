@@ -330,7 +330,8 @@ class Correlator:
                                                 ctypes.c_void_p(stream_handle)))
 
     def tuning(self):
-        """The tensor-engine setting in use: {"ksplit", "grid", "pair"}."""
+        """The tensor-engine setting that tune chose, else the default that an untuned
+        context's calls start from: {"ksplit", "grid", "pair"}."""
         k, g, p = ctypes.c_int(), ctypes.c_int(), ctypes.c_int()
         check("xgpuTuning", lib().xgpuTuning(ctypes.byref(self.ctx), ctypes.byref(k),
                                              ctypes.byref(g), ctypes.byref(p)))
