@@ -14,21 +14,21 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 SCRIPT = r"""
-import json, os, tempfile, time
+import ctypes, json, os, tempfile, time
 import torch
 from torch.profiler import profile, ProfilerActivity
 import xgpu_b200 as xg
 
-def recorded(f, times=0):
+def recorded(f, times=0, kinds=("kernel",)):
     with profile(activities=[ProfilerActivity.CUDA]) as p:
         f()
         torch.cuda.synchronize()
     path = os.path.join(tempfile.mkdtemp(), "trace.json")
     p.export_chrome_trace(path)
     with open(path) as fh:
-        ev = [e for e in json.load(fh)["traceEvents"] if e.get("cat") == "kernel"]
+        ev = [e for e in json.load(fh)["traceEvents"] if e.get("cat") in kinds]
     ev.sort(key=lambda e: e["ts"])
-    return [[e["name"].split("(")[0].split("::")[-1], e["args"]["grid"][0]] + times * [e["ts"], e["ts"] + e["dur"]]
+    return [[e["name"].split("(")[0].split("::")[-1], e["args"].get("grid", [0])[0]] + times * [e["ts"], e["ts"] + e["dur"]]
             for e in ev]
 
 def context(n, f, t, fmt="int8", **kind):
@@ -79,6 +79,15 @@ c.close()
 c, x = context(384, 64, 8192, "packed4")    # 86,016 stages of six tile rows
 out["packed chain, six rows"] = recorded(lambda: calls(c, x, 4))
 c.close()
+for skip in (0, 1):      # Complex before the output: 16-byte aligned, and not
+    c, x = context(176, 13, 32, order="rt", ntimepipe=16)
+    buf = torch.zeros(int(c.info.matLength) * 2 + 2, dtype=torch.int32, pin_memory=True)
+    c.ctx.matrix_h, c.ctx.matrix_len = buf.data_ptr(), buf.numel() // 2
+    xg.check("output", xg.lib().xgpuSetHostOutputBuffer(ctypes.byref(c.ctx)))
+    c.ctx.output_offset = skip
+    out["dump %d" % skip] = recorded(lambda: c.run_device(x.data_ptr(), xg.SYNCOP_DUMP),
+                                     kinds=("kernel", "gpu_memcpy"))
+    c.close()
 for name, kind in (("dp4a", {}), ("fp32", {"compute": "fp32", "output": "float32"})):
     c, x = context(64, 10, 1024, "dp4a_swizzled", engine="plain", **kind)
     calls(c, x, 4)
@@ -154,3 +163,11 @@ def test_small_plain_grids_come_after_their_conversion(launches, engine):
         # times in us: a few for the launch itself, where the conversion that waits for
         # the launch before takes 15 to 30
         assert launch[2] > conversion[3] - 4
+
+
+def test_narrow_stores_of_large_dumps_are_copied(launches):
+    """A register-tile dump of 6.5 MB that is 16-byte aligned goes to the host in wide
+    stores; one that is not is formatted on the device and copied."""
+    wide, narrow = ([name for name, grid in launches["dump %d" % skip]] for skip in (0, 1))
+    assert "format_host_kernel" in wide[-1]
+    assert "format_kernel" in narrow[-2] and "DtoH" in narrow[-1]
