@@ -79,6 +79,12 @@ c.close()
 c, x = context(384, 64, 8192, "packed4")    # 86,016 stages of six tile rows
 out["packed chain, six rows"] = recorded(lambda: calls(c, x, 4))
 c.close()
+c, x = context(64, 20, 1024, engine="plain", compute="fp32", output="float32")
+x.random_(-128, 128)     # two calls take the diagonal blocks' sums past 2^24
+torch.cuda.synchronize()
+out["loud"] = recorded(lambda: (calls(c, x, 6, xg.SYNCOP_SYNC_COMPUTE), c.clear(),
+                                calls(c, x, 1, xg.SYNCOP_SYNC_COMPUTE)))
+c.close()
 for skip in (0, 1):      # Complex before the output: 16-byte aligned, and not
     c, x = context(176, 13, 32, order="rt", ntimepipe=16)
     buf = torch.zeros(int(c.info.matLength) * 2 + 2, dtype=torch.int32, pin_memory=True)
@@ -171,3 +177,9 @@ def test_narrow_stores_of_large_dumps_are_copied(launches):
     wide, narrow = ([name for name, grid in launches["dump %d" % skip]] for skip in (0, 1))
     assert "format_host_kernel" in wide[-1]
     assert "format_kernel" in narrow[-2] and "DtoH" in narrow[-1]
+
+
+def test_saturated_float_sums_run_one_cta_a_block(launches):
+    names = [name for name, grid in launches["loud"]]
+    four, one = "xengine_fp32_kernel<4>", "xengine_fp32_kernel<1>"
+    assert names[0] == four and names[3:] == [one, one, one, four]

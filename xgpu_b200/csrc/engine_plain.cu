@@ -81,7 +81,15 @@ struct Params {
   int stall;        // test switch: issue no panel loads (the waits on them expire)
   int f0;           // first channel (blockIdx.y counts from it)
   int overlap;      // dp4a: may run beside the previous (adding) launch of the stream
+  FloatPast past;   // FP32 engine
 };
+
+// A block went to the float phase; the block in the middle of each channel's says so to
+// the host (fp32_pieces).
+__device__ __forceinline__ void report_past(const FloatPast &past) {
+  if (past.word && threadIdx.x == 0 && blockIdx.z == 0 && blockIdx.x == gridDim.x / 2)
+    *(volatile int *)past.word = past.integration;
+}
 
 // Queue the TMA loads of samples [tb, tb+NT) of the row panel and the column
 // panel into raw[0] / raw[1], completing on bar.  Called by one thread.  The
@@ -598,6 +606,7 @@ __device__ __forceinline__ void fp32_whole(const Params &p, uint8_t *dsm, uint32
 #pragma unroll
       for (int e = 0; e < 8; ++e) sum[e] = buffer_part(p, f, i0, j0, e);
     }
+    report_past(p.past);
     if (!float_phase<8>(p, dsm, bar0 + 16, f, rb, cb, p.t0 + ch * kTcD, 0, sum)) return;
   }
   tc::pdl_trigger();
@@ -771,6 +780,7 @@ __device__ __forceinline__ void fp32_split(const Params &p, uint8_t *dsm, uint32
   cluster_barrier();
   if (sh->past >= kFailed) return;   // the error word is set
   if (sh->past != 0) {
+    report_past(p.past);
 #pragma unroll
     for (int k = 0; k < kParts; ++k) sum[k] = buffer_part(p, f, i0, j0, e0 + k);
     if (!float_phase<kParts>(p, dsm, bar0 + 16, f, rb, cb, p.t0, e0, sum)) return;
@@ -849,12 +859,20 @@ static int plain_splits(const Sizes &s, int fcount, int tcount, bool overlap) {
 // in the exchange than it gains, unless the SMs are nearly empty.  Two pieces
 // only there: at 288 blocks they gain nothing (N=256, F=4: 55 against 52 us) and
 // the float phase loses 10%.
-static int fp32_pieces(const Sizes &s, int fcount, int tcount) {
+// past: calls of this integration went to the float phase in the middle of the array
+// (some calls ago, or none yet: it only chooses the faster way to the same sums).  There
+// each CTA converts all samples for its share of the parts, so that eight pieces never
+// pay, and four depend on how many of their CTAs come together on an SM: all sums past
+// 2^24, T=1024, us a call in chains, four pieces and one CTA a block: 84 blocks 92 and 110,
+// 96 128 and 110, 120 133 and 110, 150 (more than one whole block an SM, five CTAs of
+// the split) 136 and 161, 192 (a second wave of the split) 228 and 162.
+static int fp32_pieces(const Sizes &s, int fcount, int tcount, bool past) {
   const int sms = current_device_sms();
   const dim3 g = plain_grid(s, fcount);
   const long long blocks = (long long)g.x * g.y;
   if (tcount > 32768) return 1;
-  for (int k = 8; k > 1; k /= 2) {
+  if (past && 40 * blocks > 23LL * sms && (blocks <= sms || 4 * blocks > 5LL * sms)) return 1;
+  for (int k = past ? 4 : 8; k > 1; k /= 2) {
     const bool sparse = blocks * k <= 2LL * sms;
     const int least = k == 8 ? (sparse ? 64 : 256) : 128;
     if ((sparse || (k > 2 && 2 * blocks * k <= 11LL * sms)) && tcount / k >= least) return k;
@@ -899,6 +917,7 @@ static int plain_params(plain::Params *p, const int8_t *in, const Sizes &s, int 
   p->stall = stall;
   p->f0 = f0;
   p->overlap = 0;
+  p->past = FloatPast{};
   return 0;
 }
 
@@ -941,12 +960,12 @@ cudaError_t launch_plain_dp4a(const int8_t *in, const Sizes &s, int t0, int tcou
 
 cudaError_t launch_plain_fp32(const int8_t *in, const Sizes &s, int t0, int tcount, float *state,
                               int overwrite, cudaStream_t st, int *err, int stall, int f0,
-                              int fcount) {
+                              int fcount, const FloatPast &past) {
   if (fcount < 0) fcount = s.f - f0;
   if (f0 < 0 || fcount < 1 || f0 + fcount > s.f) return cudaErrorInvalidValue;
   cudaError_t e = plain_configure_device();
   if (e != cudaSuccess) return e;
-  const int pieces = fp32_pieces(s, fcount, tcount);
+  const int pieces = fp32_pieces(s, fcount, tcount, past.seen);
   // samples per piece: a whole number of 64-sample chunks
   int per = (tcount + pieces - 1) / pieces;
   per = (per + plain::kTcD - 1) / plain::kTcD * plain::kTcD;
@@ -954,6 +973,8 @@ cudaError_t launch_plain_fp32(const int8_t *in, const Sizes &s, int t0, int tcou
   if (plain_params(&p, in, s, t0, tcount, state, overwrite, per, err, stall, f0) != 0 ||
       make_panel_map(&p.map_float, in, s, plain::kTcF) != 0)
     return cudaErrorInvalidValue;
+  p.past = past;
+  if (past.seen) p.past.word = nullptr;   // a store over the host link ends a call 3 us later
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = plain_grid(s, fcount, pieces);
   cfg.blockDim = dim3(plain::kThreads);
@@ -967,7 +988,10 @@ cudaError_t launch_plain_fp32(const int8_t *in, const Sizes &s, int t0, int tcou
   attr[1].val.clusterDim.y = 1;
   attr[1].val.clusterDim.z = (unsigned)pieces;
   cfg.attrs = attr;
-  cfg.numAttrs = pieces > 1 ? 2 : 1;
+  // Whole blocks that come where a split call's CTAs leave room stay crowded there (the
+  // first such call 225 us for 110 at 120 blocks), so they come to an empty GPU.
+  const bool plainly = past.seen && cfg.gridDim.x * cfg.gridDim.y < 4u * current_device_sms();
+  cfg.numAttrs = pieces > 1 ? 2 : plainly ? 0 : 1;
   switch (pieces) {
     case 8: return cudaLaunchKernelEx(&cfg, plain::xengine_fp32_kernel<8>, p);
     case 4: return cudaLaunchKernelEx(&cfg, plain::xengine_fp32_kernel<4>, p);

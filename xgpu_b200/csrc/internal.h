@@ -82,9 +82,18 @@ inline Sizes compact_sizes(Sizes s) {
 cudaError_t launch_plain_dp4a(const int8_t *in, const Sizes &s, int t0, int tcount,
                               int64_t *state, int overwrite, cudaStream_t st, int *err = nullptr,
                               int stall = 0, int f0 = 0, int fcount = -1, int overlap = 0);
+// What an FP32 integration has met: its launches write `integration` to `word` (mapped
+// host memory, may be null) when float sums in the middle of the array may have passed
+// 2^24.  seen: one has.
+struct FloatPast {
+  int *word = nullptr;
+  int integration = 0;
+  bool seen = false;
+};
 cudaError_t launch_plain_fp32(const int8_t *in, const Sizes &s, int t0, int tcount,
                               float *state, int overwrite, cudaStream_t st, int *err = nullptr,
-                              int stall = 0, int f0 = 0, int fcount = -1);
+                              int stall = 0, int f0 = 0, int fcount = -1,
+                              const FloatPast &past = FloatPast{});
 
 // Tensor-core engine.  The tensor map describes `in` (see make_tc_tensor_map).
 // Launched programmatically (PDL): the prologue overlaps the previous kernel of

@@ -94,6 +94,7 @@ struct Internal {
   // (d_err is its device address) and the host reads after a wait, with no copy
   // to queue and wait for.
   int *h_err = nullptr, *d_err = nullptr;
+  int integration = 1;   // counts clears; h_err[1]: the integration last seen past 2^24 (FloatPast)
 
   cudaStream_t s_copy = nullptr, s_comp = nullptr;
   cudaStream_t s_own = nullptr;  // the context's own compute stream
@@ -387,8 +388,10 @@ int launch_engine(Internal *in, const int8_t *x, const Sizes &s, int f0, int fco
   if (wrote_state) *wrote_state = true;
   const int ow = in->state_zero ? 1 : 0;
   if (!in->int_state) {
+    const FloatPast past{in->d_err + 1, in->integration,
+                         ((volatile int *)in->h_err)[1] == in->integration};
     XGPU_CHECK(launch_plain_fp32(x, s, 0, s.t, (float *)in->d_state, ow, in->s_comp, in->d_err,
-                                 in->tune.stall, f0, fcount));
+                                 in->tune.stall, f0, fcount, past));
   } else if (in->cfg.engine == XGPU_ENGINE_PLAIN) {
     for (int t0 = 0; t0 < s.t; t0 += kSegment) {
       const int tc = s.t - t0 < kSegment ? s.t - t0 : kSegment;
@@ -860,7 +863,7 @@ int xgpuInitEx(XGPUContext *context, int device_flags, const XGPUConfig *cfg_in)
       cudaMalloc(&in->d_in[1], in_bytes) != cudaSuccess ||
       cudaMalloc(&in->d_state, state_bytes) != cudaSuccess ||
       cudaMalloc(&in->d_out, (size_t)s.mat_length * sizeof(Complex)) != cudaSuccess ||
-      cudaMallocHost(&in->h_err, sizeof(int)) != cudaSuccess ||
+      cudaMallocHost(&in->h_err, 2 * sizeof(int)) != cudaSuccess ||
       cudaHostGetDevicePointer((void **)&in->d_err, in->h_err, 0) != cudaSuccess ||
       (cfg.input_format != XGPU_INPUT_INT8 &&
        (cudaMalloc(&in->d_conv[0], (size_t)(2 * s.vec_length + 255) / 256 * 256) != cudaSuccess ||
@@ -893,7 +896,7 @@ int xgpuInitEx(XGPUContext *context, int device_flags, const XGPUConfig *cfg_in)
       return fail(XGPU_CUDA_ERROR);
     }
   }
-  *in->h_err = 0;
+  in->h_err[0] = in->h_err[1] = 0;
   if (cudaMemsetAsync(in->d_state, 0, state_bytes, in->s_comp) != cudaSuccess ||
       cudaStreamSynchronize(in->s_comp) != cudaSuccess)
     return fail(XGPU_CUDA_ERROR);
@@ -934,6 +937,7 @@ int xgpuClearDeviceIntegrationBuffer(XGPUContext *context) {
   }
   in->adding_tail = false;
   end_chain(in);
+  in->integration = in->integration < 0x7fffffff ? in->integration + 1 : 1;
   in->state_zero = true;
   return XGPU_OK;
 }
