@@ -278,9 +278,16 @@ void end_chain(Internal *in) {
   in->chain = 0;
 }
 
-// Whether everything queued on the context's own stream has finished.  Relaxed, so
-// that a capture that this thread has begun on another stream stays valid.
+// Whether everything queued on the context's own stream has finished.  A stream that
+// the program is capturing must not be asked (it counts as busy), and asking must not
+// end a capture that this thread has begun on another stream (relaxed mode).
 bool own_stream_idle(const Internal *in) {
+  cudaStreamCaptureStatus capture;
+  if (cudaStreamIsCapturing(in->s_own, &capture) != cudaSuccess ||
+      capture != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   cudaThreadExchangeStreamCaptureMode(&mode);
   const cudaError_t e = cudaStreamQuery(in->s_own);
