@@ -17,10 +17,9 @@
 //    instead of adding, so a cleared buffer is never read.
 #include <stdlib.h>
 #include <string.h>
-
-#include <chrono>
 #include <unistd.h>
 
+#include <chrono>
 #include <mutex>
 #include <new>
 
